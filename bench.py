@@ -156,9 +156,9 @@ def gen_keys(dtype: str, n: int, seed: int = 1) -> np.ndarray:
     return datagen.by_name(dtype, n, seed)
 
 
-def read_traffic(dtype: str):
+def read_traffic(kernel: str, dtype: str):
     """DRAM bytes per digit-pass launch from the committed ncu summary, if present."""
-    p = os.path.join(ROOT, "profiles", f"chunk_pass_{dtype}_256M.txt")
+    p = os.path.join(ROOT, "profiles", f"{kernel}_{dtype}_256M.txt")
     try:
         for line in open(p):
             if line.startswith("dram_bytes_per_launch="):
@@ -344,18 +344,18 @@ def run_ours(args, rank: int, world: int, local_rank: int):
     ms_per_step = total_ms / args.steps
 
     # roofline of the dominant kernel, the digit pass of whichever scheme ran (chunked:
-    # profile class "onesweep", look-back: "lookback"; with float keys both kinds are launched
-    # and the kind not chosen returns at once): algorithmic bytes per launch = one read + one
-    # write of the keys = 2 * n * w
-    chunked_ran = prof["onesweep"][1] >= prof["lookback"][1]
+    # profile class "onesweep", look-back: "lookback"): algorithmic bytes per launch = one read +
+    # one write of the keys = 2 * n * w
+    chunked_ran = prof["onesweep"][1] > prof["lookback"][1]
     os_launches, os_ms = prof["onesweep"] if chunked_ran else prof["lookback"]
     os_avg_ms = os_ms / max(1, os_launches)
     os_bytes = 2.0 * n * w
     achieved = os_bytes / (os_avg_ms / 1e3) / 1e9 if os_launches else None
-    roof = {"kernel": "chunk_pass" if chunked_ran else "onesweep_pass (look-back)", "bound": "hbm", "achieved": round(achieved, 1) if achieved else None,
+    kernel = "chunk_pass" if chunked_ran else "lookback_pass"
+    roof = {"kernel": kernel, "bound": "hbm", "achieved": round(achieved, 1) if achieved else None,
             "peak": hbm, "peak_kind": peak_kind, "unit": "GB/s",
             "frac": round(achieved / hbm, 4) if achieved else None,
-            "traffic": read_traffic(dtype), "algorithmic_bytes_per_launch": os_bytes,
+            "traffic": read_traffic(kernel, dtype), "algorithmic_bytes_per_launch": os_bytes,
             "avg_launch_ms": round(os_avg_ms, 5), "launches": os_launches}
     sort_bytes = n * w * (1 + 2 * P)
     sort_achieved = sort_bytes / (ms_per_step / 1e3) / 1e9

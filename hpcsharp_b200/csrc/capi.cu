@@ -178,10 +178,11 @@ __global__ void probe_check_kernel(const uint32_t* keys, const uint32_t* items, 
 // ranking, which is defined by PTX.  The same code generation and occupancy as a real sort: the
 // probe calls the sort's own enqueue functions.
 int probe_shipping_kernels(hpcs_ctx* ctx, int* ok) {
-  constexpr int64_t n = (int64_t(1) << 20) + 12345;
+  // the look-back passes take their middle, large and small tile at these sizes
+  constexpr int64_t sizes[3] = {(int64_t(1) << 20) + 12345, (int64_t(5) << 19) + 12345, 300007};
   uint32_t *keys = nullptr, *items = nullptr, *bad = nullptr;
-  cudaError_t e = cudaMalloc(&keys, size_t(n) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&items, size_t(n) * 4);
+  cudaError_t e = cudaMalloc(&keys, size_t(sizes[1]) * 4);
+  if (e == cudaSuccess) e = cudaMalloc(&items, size_t(sizes[1]) * 4);
   if (e == cudaSuccess) e = cudaMalloc(&bad, 4);
   if (e == cudaSuccess) e = cudaMemset(bad, 0, 4);
   int rc = e == cudaSuccess ? HPCS_OK : cuda_fail(e, "probe buffers");
@@ -189,18 +190,23 @@ int probe_shipping_kernels(hpcs_ctx* ctx, int* ok) {
   const int saved_scheme = ctx->cfg.pass_scheme;
   ctx->rank_mode = RANK_ORDERED_ATOMIC;
   cudaStream_t s = ctx->stream;
-  for (int scheme : {int(HPCS_PASSES_CHUNKED), int(HPCS_PASSES_LOOKBACK)}) {
-    ctx->cfg.pass_scheme = scheme;
+  struct Probe {
+    int scheme;
+    int64_t n;
+  };
+  for (const Probe& pr : {Probe{HPCS_PASSES_CHUNKED, sizes[0]}, Probe{HPCS_PASSES_LOOKBACK, sizes[0]},
+                          Probe{HPCS_PASSES_LOOKBACK, sizes[1]}, Probe{HPCS_PASSES_LOOKBACK, sizes[2]}}) {
+    ctx->cfg.pass_scheme = pr.scheme;
     for (uint32_t values : {20u, 3u}) {
       for (int with_items = 0; with_items < 2 && rc == HPCS_OK; with_items++) {
         uint32_t* it = with_items ? items : nullptr;
-        probe_fill_kernel<<<ctx->sms * 4, 256, 0, s>>>(keys, it, n, values);
+        probe_fill_kernel<<<ctx->sms * 4, 256, 0, s>>>(keys, it, pr.n, values);
         if ((e = cudaGetLastError()) != cudaSuccess) rc = cuda_fail(e, "probe fill");
         if (rc == HPCS_OK)
-          rc = with_items ? enqueue_sort<uint32_t, KIND_UNSIGNED, uint32_t>(ctx, keys, items, n, s)
-                          : enqueue_sort<uint32_t, KIND_UNSIGNED, NoValue>(ctx, keys, nullptr, n, s);
+          rc = with_items ? enqueue_sort<uint32_t, KIND_UNSIGNED, uint32_t>(ctx, keys, items, pr.n, s)
+                          : enqueue_sort<uint32_t, KIND_UNSIGNED, NoValue>(ctx, keys, nullptr, pr.n, s);
         if (rc == HPCS_OK) {
-          probe_check_kernel<<<ctx->sms * 4, 256, 0, s>>>(keys, it, n, bad);
+          probe_check_kernel<<<ctx->sms * 4, 256, 0, s>>>(keys, it, pr.n, bad);
           if ((e = cudaGetLastError()) != cudaSuccess) rc = cuda_fail(e, "probe check");
         }
       }
@@ -777,7 +783,7 @@ int hpcs_ctx_destroy(hpcs_ctx* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->last_stream && ctx->last_stream != ctx->stream) cudaStreamSynchronize(ctx->last_stream);
   DevBuf* bufs[] = {&ctx->keys_a, &ctx->keys_b,  &ctx->vals_a,    &ctx->vals_b, &ctx->status0,
-                    &ctx->status1, &ctx->status2, &ctx->plan, &ctx->counts, &ctx->err_accum,
+                    &ctx->status1, &ctx->plan, &ctx->counts, &ctx->err_accum,
                     &ctx->aux0,   &ctx->aux1,    &ctx->aux2};
   for (DevBuf* b : bufs)
     if (b->ptr && !b->borrowed) cudaFree(b->ptr);

@@ -19,7 +19,7 @@
 //
 // Per tile (TILE = NT x KPT keys, double-buffered by 1-D bulk async copies):
 //   rank     one ordered shared atomic per key on per-warp digit counters (or the
-//            peer-mask ranking), as in the onesweep pass;
+//            peer-mask ranking), as in the look-back pass;
 //   scan     per-digit tile totals, tile-local digit starts, per-warp offsets; the
 //            tile's global base per digit comes from the running offsets;
 //   reorder  keys into shared memory in (digit, input order) order;
@@ -88,7 +88,6 @@ __device__ __forceinline__ void chunk_pass_body(const SortArgs& args, const int 
 
   const SortPlan* plan = args.plan;
   const int pass = args.pass;
-  if (args.choose_lookback && plan->use_lookback) return;  // the look-back passes were chosen
   const int sel = plan->src_sel[pass];
   if (sel < 0) return;  // every key has the same digit here: the pass is the identity
   const int shift = 8 * pass;
@@ -135,8 +134,8 @@ __device__ __forceinline__ void chunk_pass_body(const SortArgs& args, const int 
   U* kout_base = kout;
 
   auto issue = [&](int t) {
-    onesweep_issue_tile<U, PAIRS, TILE>(smem, L::STAGE_BYTES, L::KEYS_BYTES, s_mbar, kin_c,
-                                        vin ? vin + clo : nullptr, chi - clo, t, t & 1);
+    stage_tile<U, PAIRS, TILE>(smem + size_t(t & 1) * L::STAGE_BYTES, L::KEYS_BYTES, &s_mbar[t & 1], kin_c,
+                               vin ? vin + clo : nullptr, chi - clo, t);
   };
   if (tid == 0) {
     mbar_init(&s_mbar[0], 1);

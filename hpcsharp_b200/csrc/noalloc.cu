@@ -24,7 +24,7 @@ namespace {
 // Ranking without the lane-order probe (which would need its own device memory): the fully
 // defined peer-mask ranking, 512 threads x 16 keys per tile, one CTA per SM.
 constexpr int NA_NT = 512, NA_KPT = 16, NA_TILE = NA_NT * NA_KPT;
-using NaSmem = OnesweepSmem<uint32_t, NoValue, NA_NT, NA_KPT, 2, RANK_PEER_MASK>;
+using NaSmem = LookbackSmem<uint32_t, NoValue, NA_NT, NA_KPT, RANK_PEER_MASK>;
 constexpr int64_t NA_UNITS = HPCS_NOALLOC_MAX_KEYS / NA_TILE;  // look-back units at the maximum
 
 constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
@@ -44,14 +44,12 @@ struct NaDevice {
   bool ready = false;
   unsigned char* scratch = nullptr;  // device address of g_noalloc_scratch on this device
   int sms = 0;
-  int onesweep_blocks = 1;
 };
 std::mutex g_na_mu;
 NaDevice g_na[64];
 
 #define NA_HIST_KERNEL hist_all_digits_kernel<uint32_t, KIND_UNSIGNED, HIST_NT>
-#define NA_ONESWEEP_KERNEL \
-  onesweep_pass_kernel<uint32_t, KIND_UNSIGNED, NoValue, NA_NT, NA_KPT, 2, 1, RANK_PEER_MASK, 1>
+#define NA_PASS_KERNEL lookback_pass_kernel<uint32_t, KIND_UNSIGNED, NoValue, NA_NT, NA_KPT, RANK_PEER_MASK, 8>
 
 // Once per device, with that device current.  Resolves the scratch's device address and
 // sizes the launches; clears the error word.  No allocation.
@@ -66,11 +64,8 @@ int na_setup(int dev, NaDevice** out) {
     HPCS_CUDA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
     HPCS_CUDA(cudaFuncSetAttribute(NA_HIST_KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    int(HistSmem<uint32_t>::BYTES)));
-    HPCS_CUDA(cudaFuncSetAttribute(NA_ONESWEEP_KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    HPCS_CUDA(cudaFuncSetAttribute(NA_PASS_KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    int(NaSmem::BYTES)));
-    HPCS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.onesweep_blocks, NA_ONESWEEP_KERNEL, NA_NT,
-                                                            NaSmem::BYTES));
-    if (d.onesweep_blocks < 1) d.onesweep_blocks = 1;
     HPCS_CUDA(cudaMemset(d.scratch + NA_OFF_ERR, 0, 4));
     HPCS_CUDA(cudaDeviceSynchronize());
     d.ready = true;
@@ -126,7 +121,7 @@ extern "C" int hpcs_sort_u32_dev_noalloc(uint32_t* keys, int64_t n, void* stream
   uint32_t* err = reinterpret_cast<uint32_t*>(d->scratch + NA_OFF_ERR);
 
   // The plan (counts, starts, tile counters, error bits) must start at zero on every call;
-  // K1 clears the first look-back buffer and each pass clears the other ahead of use.
+  // K1 clears the look-back passes' tile rows.
   HPCS_CUDA(cudaMemsetAsync(args.plan, 0, sizeof(SortPlan), s));
   {
     const int64_t want = (n / 4 + HIST_NT * 4 - 1) / (HIST_NT * 4);
@@ -135,11 +130,10 @@ extern "C" int hpcs_sort_u32_dev_noalloc(uint32_t* keys, int64_t n, void* stream
     HPCS_CUDA(cudaGetLastError());
   }
   {
-    const int64_t cap = int64_t(d->sms) * d->onesweep_blocks;
-    const int grid = int(units < cap ? units : cap);
+    const int grid = lookback_grid(int(units), d->sms);
     for (int p = 0; p < 4; p++) {
       args.pass = p;
-      NA_ONESWEEP_KERNEL<<<grid, NA_NT, NaSmem::BYTES, s>>>(args);
+      NA_PASS_KERNEL<<<grid, NA_NT, NaSmem::BYTES, s>>>(args);
       HPCS_CUDA(cudaGetLastError());
     }
   }

@@ -9,7 +9,7 @@
 // order of the keys, the CTA reads its segment once to histogram every digit, then runs each
 // 8-bit pass tile by tile with running per-digit offsets: tiles of one segment are processed
 // in order by one CTA, so no look-back between CTAs is needed and every pass is one read and
-// one write (the onesweep's 36 B/key for 32-bit keys).  Segments that fit in one tile are
+// one write (36 B/key for 32-bit keys).  Segments that fit in one tile are
 // sorted entirely in shared memory: one global read, all passes in shared memory, one
 // global write.  Ranking is the sort's in-warp ranking (ordered shared atomics after the
 // lane-order probe, or the peer-mask ranking).

@@ -11,6 +11,7 @@
 
 #include "../../include/hpcs_gpu.h"
 #include "chunk_pass.cuh"
+#include "lookback_pass.cuh"
 #include "radix_kernels.cuh"
 #include "small_sort.cuh"
 
@@ -64,7 +65,6 @@ struct hpcs_ctx {
   std::vector<cudaEvent_t> event_pool;
   // scratch
   hpcs::DevBuf keys_a, keys_b, vals_a, vals_b, status0, status1, plan, counts, err_accum;
-  hpcs::DevBuf status2;  // second look-back buffer when the device chooses the scheme
   hpcs::DevBuf aux0, aux1, aux2;
   // pinned ring and copy threads for host arrays in pageable memory (host_copy.cuh)
   hpcs::HostStager* stager = nullptr;
@@ -97,44 +97,59 @@ struct KernelTimer {
 int enter_stream(hpcs_ctx* ctx, cudaStream_t s);
 uint32_t* device_error_word(hpcs_ctx* ctx);
 
+// Look-back tile shapes: threads, keys per thread of the large tile, keys per thread whose shared
+// accesses are in flight together.  The large tile fills the two tile buffers (a tile costs ~1600
+// clocks of barriers and latency whatever its size: u32 keys 2^28, us per pass: 40 keys 592, 32 keys
+// 650, 24 keys 703, 16 keys 953; 42 no better than 40).  The peer-mask ranking's 32 KiB of lane masks
+// leave less room.  The 32-bit keys-only shape can be overridden at build time.
+#ifndef HPCS_K32_KPT
+#define HPCS_K32_KPT 40
+#endif
 template <class U, class V, int MODE>
 struct SortConfig;
-// Tile shapes (threads x keys per thread), prefetch stages, CTAs per SM and CTAs per
-// look-back unit (cluster size), per key/payload type and ranking mode.  The 32-bit
-// keys-only shape of the ordered-atomic ranking can be overridden at build time for
-// tuning sweeps.
-#ifndef HPCS_K32_NT
-#define HPCS_K32_NT 1024
-#endif
-#ifndef HPCS_K32_KPT
-#define HPCS_K32_KPT 16
-#endif
-#ifndef HPCS_K32_MINB
-#define HPCS_K32_MINB 1
-#endif
-#ifndef HPCS_CL
-#define HPCS_CL 1
-#endif
 template <>
 struct SortConfig<uint32_t, NoValue, RANK_ORDERED_ATOMIC> {
-  static constexpr int NT = HPCS_K32_NT, KPT = HPCS_K32_KPT, STAGES = 2, MINB = HPCS_K32_MINB, CL = HPCS_CL;
+  static constexpr int NT = 512, KPT = HPCS_K32_KPT, BATCH = 8;
 };
 template <>
-struct SortConfig<uint32_t, NoValue, RANK_PEER_MASK> {  // + 32 KiB of lane masks
-  static constexpr int NT = 512, KPT = 16, STAGES = 2, MINB = 1, CL = 1;
+struct SortConfig<uint64_t, NoValue, RANK_ORDERED_ATOMIC> {
+  static constexpr int NT = 512, KPT = 24, BATCH = 4;
 };
-template <int MODE>
-struct SortConfig<uint64_t, NoValue, MODE> {
-  static constexpr int NT = 512, KPT = 8, STAGES = 2, MINB = 2, CL = HPCS_CL;
+template <>
+struct SortConfig<uint32_t, uint32_t, RANK_ORDERED_ATOMIC> {
+  static constexpr int NT = 512, KPT = 24, BATCH = 8;
 };
-template <int MODE>
-struct SortConfig<uint32_t, uint32_t, MODE> {
-  static constexpr int NT = 512, KPT = 8, STAGES = 2, MINB = 2, CL = HPCS_CL;
+template <>
+struct SortConfig<uint64_t, uint32_t, RANK_ORDERED_ATOMIC> {
+  static constexpr int NT = 512, KPT = 16, BATCH = 8;
 };
-template <int MODE>
-struct SortConfig<uint64_t, uint32_t, MODE> {
-  static constexpr int NT = 512, KPT = 6, STAGES = 2, MINB = 2, CL = HPCS_CL;
+template <>
+struct SortConfig<uint32_t, NoValue, RANK_PEER_MASK> {
+  static constexpr int NT = 512, KPT = 32, BATCH = 8;
 };
+template <>
+struct SortConfig<uint64_t, NoValue, RANK_PEER_MASK> {
+  static constexpr int NT = 512, KPT = 16, BATCH = 4;
+};
+template <>
+struct SortConfig<uint32_t, uint32_t, RANK_PEER_MASK> {
+  static constexpr int NT = 512, KPT = 16, BATCH = 8;
+};
+template <>
+struct SortConfig<uint64_t, uint32_t, RANK_PEER_MASK> {
+  static constexpr int NT = 512, KPT = 12, BATCH = 4;
+};
+// Keys per thread of the tile a sort of n keys takes: 8 while one such tile per SM holds the keys, 16
+// up to two tiles per SM, then the large tile.  Smaller tiles put more SMs to work and their passes
+// are shorter chains (u32 pass, us, 8 / 16 / 40 keys: 300 Ki keys 12.8 / 12.8 / 20.9, 1 Mi 16.7 / 15.0
+// / 21.0, 3 M 27.1 / 20.8 / 21.2, 10 M 68 / 43.7 / 35.6).  The peer-mask ranking has one tile.
+template <class U, class V, int MODE>
+inline int lookback_kpt(int64_t n, int sms) {
+  using C = SortConfig<U, V, MODE>;
+  if (MODE == RANK_PEER_MASK) return C::KPT;
+  if (n <= int64_t(sms) * C::NT * 8) return 8;
+  return n <= int64_t(2) * sms * C::NT * 16 ? 16 : C::KPT;
+}
 
 // Chunked-pass tile shapes (threads x keys per thread).  Every shape keeps its two stage
 // buffers within 128 KiB, which leaves room for 148 ranges x 512 bytes of next-digit
@@ -191,29 +206,6 @@ struct ChunkConfig<uint64_t, uint32_t, RANK_PEER_MASK> {
 };
 constexpr size_t MAX_DYN_SMEM = 232448;  // 227 KiB per CTA on sm_100
 
-// Automatic scheme: below these sizes the look-back passes were measured faster on B200 (the
-// chunked passes' per-range count tables cost about J^2 x 256 global adds per pass, which
-// small sorts do not amortise).  u32 keys: equal at 32 Mi, chunked 2% ahead at 64 Mi;
-// u64 keys and u32 pairs: chunked ahead from 8 Mi; u64 + u32 pairs: from 4 Mi.
-template <class U, class V>
-struct ChunkMinKeys;
-template <>
-struct ChunkMinKeys<uint32_t, NoValue> {
-  static constexpr int64_t value = int64_t(48) << 20;
-};
-template <>
-struct ChunkMinKeys<uint64_t, NoValue> {
-  static constexpr int64_t value = int64_t(6) << 20;
-};
-template <>
-struct ChunkMinKeys<uint32_t, uint32_t> {
-  static constexpr int64_t value = int64_t(6) << 20;
-};
-template <>
-struct ChunkMinKeys<uint64_t, uint32_t> {
-  static constexpr int64_t value = int64_t(3) << 20;
-};
-
 template <class U, class V, int MODE>
 struct ChunkShape {
   using C = ChunkConfig<U, V, MODE>;
@@ -222,19 +214,29 @@ struct ChunkShape {
   static constexpr int MAX_RANGES = 2 * int((MAX_DYN_SMEM - L::BASE_BYTES) / (RADIX * 4));
 };
 
+// Launches kernel k; chained: as a programmatic dependent of the kernel before it on the stream (k
+// calls chain_wait before it touches memory).
+template <class... P, class... A>
+cudaError_t launch_chained(bool chained, void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s, A... a) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(grid), 1, 1);
+  cfg.blockDim = dim3(unsigned(block), 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k, a...);
+}
+
 constexpr int HIST_NT = 1024;
 
 // Launches K1 (one CTA per SM, 128 KiB of lane-private counters).
 template <class U, int KIND>
 int launch_histogram(hpcs_ctx* ctx, const U* keys, int64_t n, uint32_t* hist_out, const SortArgs& args,
                      int make_plan, cudaStream_t s);
-
-template <class Kernel>
-int occupancy_blocks(Kernel k, int nt, size_t smem) {
-  int blocks = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, nt, smem) != cudaSuccess) return 1;
-  return blocks > 0 ? blocks : 1;
-}
 
 template <class U, int KIND>
 int launch_histogram(hpcs_ctx* ctx, const U* keys, int64_t n, uint32_t* hist_out, const SortArgs& args,
@@ -254,44 +256,44 @@ int launch_histogram(hpcs_ctx* ctx, const U* keys, int64_t n, uint32_t* hist_out
   return HPCS_OK;
 }
 
-// Onesweep launches for every digit pass, with the context's ranking mode.  Persistent
-// grid of as many CL-CTA clusters as fit on the GPU at once.
-template <class U, int KIND, class V, int MODE>
-int launch_onesweep_passes(hpcs_ctx* ctx, SortArgs args, cudaStream_t s) {
+// CTAs of a look-back pass: a persistent grid of one CTA per SM, one of them the scanner, at most
+// one per tile besides it; a single tile needs no scanner.
+inline int lookback_grid(int num_tiles, int sms) {
+  const int want = num_tiles > 1 ? num_tiles + 1 : 1;
+  return want < sms ? want : (sms > 1 ? sms : 2);
+}
+
+// Look-back launches for every digit pass, with tiles of KPT keys per thread.
+template <class U, int KIND, class V, int MODE, int KPT>
+int launch_lookback_tiles(hpcs_ctx* ctx, SortArgs args, bool chained, cudaStream_t s) {
   using C = SortConfig<U, V, MODE>;
-  using L = OnesweepSmem<U, V, C::NT, C::KPT, C::STAGES, MODE>;
+  using L = LookbackSmem<U, V, C::NT, KPT, MODE>;
+  static_assert(L::BYTES <= MAX_DYN_SMEM, "two tile buffers fit");
   constexpr int P = int(sizeof(U));
-  auto k = onesweep_pass_kernel<U, KIND, V, C::NT, C::KPT, C::STAGES, C::MINB, MODE, C::CL>;
-  static int clusters_by_dev[64] = {0};
-  int& clusters = clusters_by_dev[ctx->device & 63];
-  cudaLaunchConfig_t cfg{};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = C::CL;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.blockDim = dim3(C::NT, 1, 1);
-  cfg.dynamicSmemBytes = L::BYTES;
-  cfg.stream = s;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (!clusters) {
+  auto k = lookback_pass_kernel<U, KIND, V, C::NT, KPT, MODE, C::BATCH>;
+  static int attr_set[64] = {0};
+  if (!attr_set[ctx->device & 63]) {
     HPCS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(L::BYTES)));
-    if (C::CL > 1) HPCS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 0));
-    cfg.gridDim = dim3(C::CL * ctx->sms, 1, 1);
-    int mc = 0;
-    HPCS_CUDA(cudaOccupancyMaxActiveClusters(&mc, k, &cfg));
-    clusters = mc > 0 ? mc : 1;
+    attr_set[ctx->device & 63] = 1;
   }
-  const int64_t units = args.num_tiles;
-  const int grid_clusters = int(units < clusters ? units : clusters);
-  cfg.gridDim = dim3(grid_clusters * C::CL, 1, 1);
+  const int grid = lookback_grid(args.num_tiles, ctx->sms);
   for (int p = 0; p < P; p++) {
     args.pass = p;
     KernelTimer kt(ctx, s, HPCS_K_LOOKBACK);
-    HPCS_CUDA(cudaLaunchKernelEx(&cfg, k, args));
+    HPCS_CUDA(launch_chained(chained, k, grid, C::NT, L::BYTES, s, args));
   }
   return HPCS_OK;
+}
+
+template <class U, int KIND, class V, int MODE>
+int launch_lookback_passes(hpcs_ctx* ctx, const SortArgs& args, bool chained, cudaStream_t s) {
+  constexpr int LARGE = SortConfig<U, V, MODE>::KPT;
+  constexpr bool ONE = MODE == RANK_PEER_MASK;
+  switch (lookback_kpt<U, V, MODE>(args.n, ctx->sms)) {
+    case 8: return launch_lookback_tiles<U, KIND, V, MODE, ONE ? LARGE : 8>(ctx, args, chained, s);
+    case 16: return launch_lookback_tiles<U, KIND, V, MODE, ONE ? LARGE : 16>(ctx, args, chained, s);
+    default: return launch_lookback_tiles<U, KIND, V, MODE, LARGE>(ctx, args, chained, s);
+  }
 }
 
 // Chunked digit passes: one CTA per key range, one launch per digit.
@@ -371,23 +373,21 @@ int enqueue_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t
   if (n > MAX_KEYS_PER_SORT) return fail(HPCS_ERR_RANGE, "n exceeds HPCS_MAX_KEYS");
   // small sorts: one cooperative launch (not inside a stream capture, and not when a pass
   // scheme is forced)
-  if (n <= SMALL_MAX_KEYS && ctx->cfg.pass_scheme == HPCS_PASSES_AUTO) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    HPCS_CUDA(cudaStreamIsCapturing(s, &cap));
-    if (cap == cudaStreamCaptureStatusNone) return enqueue_small_sort<U, KIND, V>(ctx, keys, vals, n, s);
-  }
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  HPCS_CUDA(cudaStreamIsCapturing(s, &cap));
+  const bool capturing = cap != cudaStreamCaptureStatusNone;
+  if (n <= SMALL_MAX_KEYS && ctx->cfg.pass_scheme == HPCS_PASSES_AUTO && !capturing)
+    return enqueue_small_sort<U, KIND, V>(ctx, keys, vals, n, s);
   if (ctx->cfg.pass_scheme == HPCS_PASSES_LOOKBACK && n > MAX_KEYS_LOOKBACK)
     return fail(HPCS_ERR_RANGE, "look-back passes take at most 2^30 - 1 keys (30-bit prefixes)");
-  const bool lookback = ctx->cfg.pass_scheme == HPCS_PASSES_LOOKBACK ||
-                        (ctx->cfg.pass_scheme != HPCS_PASSES_CHUNKED && n < ChunkMinKeys<U, V>::value);
-  // 4-byte float keys without items, AUTO scheme, large sorts: K1 picks the scheme from the
-  // digit counts (normally distributed floats sort faster with the look-back passes, floats
-  // with a dominant exponent with the chunked ones).  Not on borrowed (serving) scratch.
-  const bool choose = !lookback && ctx->cfg.pass_scheme == HPCS_PASSES_AUTO && KIND == KIND_FLOAT &&
-                      sizeof(U) == 4 && !PAIRS && n <= MAX_KEYS_LOOKBACK && !ctx->status1.borrowed;
+  const bool lookback = ctx->cfg.pass_scheme != HPCS_PASSES_CHUNKED;
+  // the look-back launches are chained: each pass's CTAs start as the last pass's finish (u32 sorts,
+  // us, plain / chained launches: 150 Ki keys 69 / 51, 1 Mi 75 / 61, 10 M 181 / 167)
+  const bool chained = lookback && !capturing;
   const bool ordered = ctx->rank_mode == RANK_ORDERED_ATOMIC;
-  const int64_t unit = ordered ? int64_t(CA::NT) * CA::KPT * CA::CL : int64_t(CP::NT) * CP::KPT * CP::CL;
-  const int64_t num_tiles = lookback || choose ? (n + unit - 1) / unit : 0;  // look-back units
+  const int64_t unit = ordered ? int64_t(CA::NT) * lookback_kpt<U, V, RANK_ORDERED_ATOMIC>(n, ctx->sms)
+                               : int64_t(CP::NT) * lookback_kpt<U, V, RANK_PEER_MASK>(n, ctx->sms);
+  const int64_t num_tiles = lookback ? (n + unit - 1) / unit : 0;
   ChunkGeometry geo{0, 0, 0};
   if (!lookback) {
     using SA = ChunkShape<U, V, RANK_ORDERED_ATOMIC>;
@@ -418,9 +418,6 @@ int enqueue_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t
   const size_t status_bytes = lookback ? size_t(num_tiles) * RADIX * 4 : size_t(geo.chunks) * (P + 3) * RADIX * 4;
   if ((rc = ensure(ctx, ctx->status0, status_bytes)) != HPCS_OK) return rc;
   if (lookback && (rc = ensure(ctx, ctx->status1, status_bytes)) != HPCS_OK) return rc;
-  const size_t lb_bytes = size_t(num_tiles) * RADIX * 4;  // one look-back buffer (choose)
-  if (choose && (rc = ensure(ctx, ctx->status1, lb_bytes)) != HPCS_OK) return rc;
-  if (choose && (rc = ensure(ctx, ctx->status2, lb_bytes)) != HPCS_OK) return rc;
   if ((rc = ensure(ctx, ctx->plan, sizeof(SortPlan))) != HPCS_OK) return rc;
 
   SortArgs args{};
@@ -447,15 +444,6 @@ int enqueue_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t
     args.chunk_keys = geo.chunk_keys;
     args.chunk_magic = geo.magic;
   }
-  if (choose) {
-    // the look-back passes' buffers are status1 and status2; K1 (chunked mode) does not
-    // zero the first one, so it is cleared here
-    args.choose_lookback = 1;
-    args.status[0] = static_cast<uint32_t*>(ctx->status1.ptr);
-    args.status[1] = static_cast<uint32_t*>(ctx->status2.ptr);
-    HPCS_CUDA(cudaMemsetAsync(args.status[0], 0, lb_bytes, s));
-  }
-
   HPCS_CUDA(cudaMemsetAsync(args.plan, 0, sizeof(SortPlan), s));
 
   // K1: fused histogram + plan
@@ -463,21 +451,20 @@ int enqueue_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t
     KernelTimer kt(ctx, s, HPCS_K_HISTOGRAM);
     if ((rc = launch_histogram<U, KIND>(ctx, a, n, &args.plan->hist[0][0], args, 1, s)) != HPCS_OK) return rc;
   }
-  // K3: one launch per digit (with `choose`, both kinds; the ones K1 did not choose return)
+  // K3: one launch per digit
   if (!lookback)
     rc = ordered ? launch_chunk_passes<U, KIND, V, RANK_ORDERED_ATOMIC>(ctx, args, s)
                  : launch_chunk_passes<U, KIND, V, RANK_PEER_MASK>(ctx, args, s);
-  if (rc == HPCS_OK && (lookback || choose))
-    rc = ordered ? launch_onesweep_passes<U, KIND, V, RANK_ORDERED_ATOMIC>(ctx, args, s)
-                 : launch_onesweep_passes<U, KIND, V, RANK_PEER_MASK>(ctx, args, s);
+  else
+    rc = ordered ? launch_lookback_passes<U, KIND, V, RANK_ORDERED_ATOMIC>(ctx, args, chained, s)
+                 : launch_lookback_passes<U, KIND, V, RANK_PEER_MASK>(ctx, args, chained, s);
   if (rc != HPCS_OK) return rc;
   // finalize: result back into the caller's buffer if it ended in B; collect errors
   {
     int64_t want = (n + 255) / 256;
     int grid = int(want > int64_t(ctx->sms) * 8 ? int64_t(ctx->sms) * 8 : want);
     KernelTimer kt(ctx, s, HPCS_K_FINALIZE);
-    finalize_kernel<U><<<grid, 256, 0, s>>>(args, PAIRS ? 1 : 0, device_error_word(ctx));
-    HPCS_CUDA(cudaGetLastError());
+    HPCS_CUDA(launch_chained(chained, finalize_kernel<U>, grid, 256, 0, s, args, PAIRS ? 1 : 0, device_error_word(ctx)));
   }
   if (keys_unaligned)
     HPCS_CUDA(cudaMemcpyAsync(keys, a, size_t(n) * sizeof(U), cudaMemcpyDeviceToDevice, s));
