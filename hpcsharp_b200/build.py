@@ -26,7 +26,8 @@ NVCC_FLAGS = [
 ]
 OBJ_DIR = os.path.join(ROOT, "_build")
 
-GPU_SOURCES = ["capi.cu", "noalloc.cu", "segmented_host.cu", "serve.cu"]
+GPU_SOURCES = ["capi.cu", "noalloc.cu", "segmented_host.cu", "serve.cu", "sort_u32.cu", "sort_u64.cu", "pairs_u32.cu",
+               "pairs_u64.cu"]
 
 
 def _gpu_deps() -> list[str]:

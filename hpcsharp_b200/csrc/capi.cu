@@ -212,7 +212,7 @@ int probe_shipping_kernels(hpcs_ctx* ctx, int* ok) {
       }
     }
   }
-  // the one-launch sort of small arrays (small_sort.cuh), taken by the default scheme
+  // the one-launch sort of small arrays (cluster_sort.cuh), taken by the default scheme
   ctx->cfg.pass_scheme = HPCS_PASSES_AUTO;
   constexpr int64_t n_small = 100003;
   for (uint32_t values : {20u, 3u}) {

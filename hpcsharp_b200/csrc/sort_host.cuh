@@ -11,9 +11,9 @@
 
 #include "../../include/hpcs_gpu.h"
 #include "chunk_pass.cuh"
+#include "cluster_sort.cuh"
 #include "lookback_pass.cuh"
 #include "radix_kernels.cuh"
-#include "small_sort.cuh"
 
 namespace hpcs {
 
@@ -335,34 +335,67 @@ inline ChunkGeometry chunk_geometry(int64_t n, int tile, int max_ranges) {
   return g;
 }
 
-// Enqueue a full LSD sort of n keys (and optional 4-byte items) in device memory.
-// A sort of at most SMALL_MAX_KEYS keys (and items) in one cooperative launch (small_sort.cuh),
-// with the context's ranking mode; scratch: B, the per-CTA digit totals and the barrier words.
-template <class U, int KIND, class V>
-int enqueue_small_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t s) {
-  constexpr bool PAIRS = !std::is_same<V, NoValue>::value;
-  const int G = int((n + SMALL_TILE - 1) / SMALL_TILE);
-  int rc;
-  if ((rc = ensure(ctx, ctx->keys_b, size_t(n) * sizeof(U))) != HPCS_OK) return rc;
-  if (PAIRS && (rc = ensure(ctx, ctx->vals_b, size_t(n) * 4)) != HPCS_OK) return rc;
-  uint32_t* vb = PAIRS ? static_cast<uint32_t*>(ctx->vals_b.ptr) : nullptr;
-  if ((rc = ensure(ctx, ctx->status0, (size_t(G) * RADIX + 2) * 4)) != HPCS_OK) return rc;
-  U* b = static_cast<U*>(ctx->keys_b.ptr);
-  uint32_t* counts = static_cast<uint32_t*>(ctx->status0.ptr);
-  uint32_t* bar = counts + size_t(G) * RADIX;
-  uint32_t* err = device_error_word(ctx);
-  int n32 = int(n);
-  uint64_t spin = uint64_t(ctx->cfg.spin_limit_ns);
-  HPCS_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(uint32_t), s));
-  void* args[] = {&keys, &b, &vals, &vb, &n32, &counts, &bar, &err, &spin};
-  const void* k = ctx->rank_mode == RANK_ORDERED_ATOMIC
-                      ? reinterpret_cast<const void*>(small_sort_kernel<U, KIND, V, RANK_ORDERED_ATOMIC>)
-                      : reinterpret_cast<const void*>(small_sort_kernel<U, KIND, V, RANK_PEER_MASK>);
+// Slice shapes of the one-launch small sort, in keys per thread.  One slice up to 8192 keys, with the
+// smallest of 4, 8 and 16 that holds them (u32 keys, us per call: 1000 keys 6.3 / 8.3 / 10.4, 4096 keys
+// 14.5 (two slices) / 8.3 / 12.4; 16384 keys in one slice of 32 per thread 22.7, in four of 8 18.6);
+// beyond, the smallest of 8, 16 and (32-bit keys alone) 32 of which 16 slices hold them: fewer keys per
+// CTA make shorter passes (65536 keys 20.6 / 24.7 / 39.0, 131072 keys - / 26.8 / 39.3, 262144 keys 41.1
+// with 32, 52 on the look-back passes).  The peer-mask ranking has one shape.
+constexpr int64_t CS_SOLO_KEYS = 8192;
+
+// Launches the one-launch small sort with KPT keys per thread if n fits (else *done stays false).  The
+// cluster is the next power of two of CTAs; more than 8 where the device schedules such clusters.
+template <class U, int KIND, class V, int MODE, int KPT>
+int launch_cluster_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t s, bool* done) {
+  using L = ClusterSmem<U, V, KPT, MODE>;
+  static_assert(L::BYTES <= MAX_DYN_SMEM, "a slice fits");
+  auto k = cluster_sort_kernel<U, KIND, V, KPT, MODE>;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.blockDim = dim3(CS_NT, 1, 1);
+  cfg.dynamicSmemBytes = L::BYTES;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  static int max_ctas_by_dev[64] = {0};
+  int& max_ctas = max_ctas_by_dev[ctx->device & 63];
+  if (!max_ctas) {
+    HPCS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(L::BYTES)));
+    HPCS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    attr.val.clusterDim.x = CS_MAX_CTAS;
+    cfg.gridDim = dim3(CS_MAX_CTAS, 1, 1);
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess) cudaGetLastError();
+    max_ctas = clusters > 0 ? CS_MAX_CTAS : 8;
+  }
+  int ctas = 1;
+  while (int64_t(ctas) * L::SLICE < n) ctas *= 2;
+  if (ctas > max_ctas) return HPCS_OK;
+  attr.val.clusterDim.x = unsigned(ctas);
+  cfg.gridDim = dim3(unsigned(ctas), 1, 1);
   KernelTimer kt(ctx, s, HPCS_K_LOOKBACK);
-  HPCS_CUDA(cudaLaunchCooperativeKernel(k, dim3(G), dim3(SMALL_NT), args, 0, s));
+  HPCS_CUDA(cudaLaunchKernelEx(&cfg, k, keys, vals, uint32_t(n), int(ctx->cfg.skip_trivial_passes), device_error_word(ctx)));
+  *done = true;
   return HPCS_OK;
 }
 
+// A small sort in one cluster launch if n fits (else *done stays false).
+template <class U, int KIND, class V, int MODE>
+int enqueue_cluster_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t s, bool* done) {
+  constexpr bool ONE = MODE == RANK_PEER_MASK;
+  constexpr int LARGEST = !ONE && sizeof(U) == 4 && std::is_same<V, NoValue>::value ? 32 : 16;
+  const int64_t per = n <= CS_SOLO_KEYS ? n : (n + CS_MAX_CTAS - 1) / CS_MAX_CTAS;  // keys a slice must hold
+  if (per <= CS_NT * 4 && n <= CS_SOLO_KEYS) return launch_cluster_sort<U, KIND, V, MODE, ONE ? 16 : 4>(ctx, keys, vals, n, s, done);
+  if (per <= CS_NT * 8) return launch_cluster_sort<U, KIND, V, MODE, ONE ? 16 : 8>(ctx, keys, vals, n, s, done);
+  if (per <= CS_NT * 16) return launch_cluster_sort<U, KIND, V, MODE, 16>(ctx, keys, vals, n, s, done);
+  if (per <= CS_NT * LARGEST) return launch_cluster_sort<U, KIND, V, MODE, LARGEST>(ctx, keys, vals, n, s, done);
+  return HPCS_OK;
+}
+
+// Enqueue a full LSD sort of n keys (and optional 4-byte items) in device memory.
 // keys/vals are sorted in place (with scratch B owned by the context).
 template <class U, int KIND, class V>
 int enqueue_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t s) {
@@ -371,20 +404,26 @@ int enqueue_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t
   constexpr bool PAIRS = !std::is_same<V, NoValue>::value;
   if (n <= 1) return HPCS_OK;
   if (n > MAX_KEYS_PER_SORT) return fail(HPCS_ERR_RANGE, "n exceeds HPCS_MAX_KEYS");
-  // small sorts: one cooperative launch (not inside a stream capture, and not when a pass
-  // scheme is forced)
+  if (ctx->cfg.pass_scheme == HPCS_PASSES_LOOKBACK && n > MAX_KEYS_LOOKBACK)
+    return fail(HPCS_ERR_RANGE, "look-back passes take at most 2^30 - 1 keys when forced");
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   HPCS_CUDA(cudaStreamIsCapturing(s, &cap));
   const bool capturing = cap != cudaStreamCaptureStatusNone;
-  if (n <= SMALL_MAX_KEYS && ctx->cfg.pass_scheme == HPCS_PASSES_AUTO && !capturing)
-    return enqueue_small_sort<U, KIND, V>(ctx, keys, vals, n, s);
-  if (ctx->cfg.pass_scheme == HPCS_PASSES_LOOKBACK && n > MAX_KEYS_LOOKBACK)
-    return fail(HPCS_ERR_RANGE, "look-back passes take at most 2^30 - 1 keys (30-bit prefixes)");
+  const bool ordered = ctx->rank_mode == RANK_ORDERED_ATOMIC;
+  int rc;
+  if ((rc = ensure(ctx, ctx->keys_b, size_t(n) * sizeof(U))) != HPCS_OK) return rc;
+  if (PAIRS && (rc = ensure(ctx, ctx->vals_b, size_t(n) * 4)) != HPCS_OK) return rc;
+  // small sorts: one cluster launch (not when a pass scheme is forced)
+  if (ctx->cfg.pass_scheme == HPCS_PASSES_AUTO) {
+    bool done = false;
+    rc = ordered ? enqueue_cluster_sort<U, KIND, V, RANK_ORDERED_ATOMIC>(ctx, keys, vals, n, s, &done)
+                 : enqueue_cluster_sort<U, KIND, V, RANK_PEER_MASK>(ctx, keys, vals, n, s, &done);
+    if (rc != HPCS_OK || done) return rc;
+  }
   const bool lookback = ctx->cfg.pass_scheme != HPCS_PASSES_CHUNKED;
   // the look-back launches are chained: each pass's CTAs start as the last pass's finish (u32 sorts,
   // us, plain / chained launches: 150 Ki keys 69 / 51, 1 Mi 75 / 61, 10 M 181 / 167)
   const bool chained = lookback && !capturing;
-  const bool ordered = ctx->rank_mode == RANK_ORDERED_ATOMIC;
   const int64_t unit = ordered ? int64_t(CA::NT) * lookback_kpt<U, V, RANK_ORDERED_ATOMIC>(n, ctx->sms)
                                : int64_t(CP::NT) * lookback_kpt<U, V, RANK_PEER_MASK>(n, ctx->sms);
   const int64_t num_tiles = lookback ? (n + unit - 1) / unit : 0;
@@ -401,9 +440,6 @@ int enqueue_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t
   uint32_t* va = vals;
   const bool keys_unaligned = (reinterpret_cast<uintptr_t>(keys) & 15) != 0;
   const bool vals_unaligned = PAIRS && (reinterpret_cast<uintptr_t>(vals) & 15) != 0;
-  int rc;
-  if ((rc = ensure(ctx, ctx->keys_b, size_t(n) * sizeof(U))) != HPCS_OK) return rc;
-  if (PAIRS && (rc = ensure(ctx, ctx->vals_b, size_t(n) * 4)) != HPCS_OK) return rc;
   if (keys_unaligned) {
     if ((rc = ensure(ctx, ctx->keys_a, size_t(n) * sizeof(U))) != HPCS_OK) return rc;
     a = static_cast<U*>(ctx->keys_a.ptr);
@@ -471,5 +507,19 @@ int enqueue_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t
   if (vals_unaligned) HPCS_CUDA(cudaMemcpyAsync(vals, va, size_t(n) * 4, cudaMemcpyDeviceToDevice, s));
   return HPCS_OK;
 }
+
+// Instantiated once each (sort_u32.cu, sort_u64.cu, pairs_u32.cu, pairs_u64.cu).
+#ifndef HPCS_INSTANTIATE_SORTS
+#define HPCS_EXTERN_SORT(U, KIND)                                                               \
+  extern template int enqueue_sort<U, KIND, NoValue>(hpcs_ctx*, U*, uint32_t*, int64_t, cudaStream_t); \
+  extern template int enqueue_sort<U, KIND, uint32_t>(hpcs_ctx*, U*, uint32_t*, int64_t, cudaStream_t);
+HPCS_EXTERN_SORT(uint32_t, KIND_UNSIGNED)
+HPCS_EXTERN_SORT(uint32_t, KIND_SIGNED)
+HPCS_EXTERN_SORT(uint32_t, KIND_FLOAT)
+HPCS_EXTERN_SORT(uint64_t, KIND_UNSIGNED)
+HPCS_EXTERN_SORT(uint64_t, KIND_SIGNED)
+HPCS_EXTERN_SORT(uint64_t, KIND_FLOAT)
+#undef HPCS_EXTERN_SORT
+#endif
 
 }  // namespace hpcs

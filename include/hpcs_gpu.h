@@ -80,8 +80,8 @@ typedef struct hpcs_config {
   int64_t spin_limit_ns;       /* bound on every device-side wait (default 2e9) */
   int32_t poison_tile;         /* test hook: tile whose device wait times out (-1 = off) */
   int32_t pass_scheme;         /* digit passes: HPCS_PASSES_AUTO (0, default): up to 131072
-                                  keys every pass in one cooperative launch (outside stream
-                                  capture), else the single-sweep look-back passes;
+                                  keys (262144 4-byte keys without items) every pass in one
+                                  cluster launch, else the single-sweep look-back passes;
                                   HPCS_PASSES_LOOKBACK (1): the look-back passes for every size
                                   up to 2^30 - 1 keys; HPCS_PASSES_CHUNKED (2): per-range counts
                                   from the previous pass, no inter-CTA waiting */
