@@ -477,10 +477,8 @@ int select_topk_dev(hpcs_ctx* ctx, T* a, int64_t n, int64_t k, void* stream) {
   U* d = reinterpret_cast<U*>(a);
   U* o = static_cast<U*>(ctx->keys_b.ptr);
   SelectState* st = nullptr;
-  if ((rc = enqueue_select<U, KIND>(ctx, d, n, k, s, &st)) != HPCS_OK) return rc;
-  if ((rc = enqueue_partition<U, KIND>(ctx, d, n, st, o, s)) != HPCS_OK) return rc;
-  HPCS_CUDA(cudaMemcpyAsync(d, o, size_t(n) * sizeof(U), cudaMemcpyDeviceToDevice, s));
-  return HPCS_OK;
+  if ((rc = enqueue_select<U, KIND>(ctx, d, n, k, s, &st, o)) != HPCS_OK) return rc;
+  return enqueue_partition<U, KIND>(ctx, o, n, st, d, s);
 }
 
 // ---- PartitionRadix / SelectRadix(Par) ---------------------------------------------------
@@ -517,9 +515,8 @@ int enqueue_partition_ranks(hpcs_ctx* ctx, U* d, U* o, int64_t n, const std::vec
   for (int64_t rank : r) {
     if (rank < lo) continue;  // inside the previous rank's run of keys equal to its key
     SelectState* st = nullptr;
-    if ((rc = enqueue_select<U, KIND>(ctx, d + lo, n - lo, rank - lo, s, &st)) != HPCS_OK) return rc;
-    if ((rc = enqueue_partition<U, KIND>(ctx, d + lo, n - lo, st, o + lo, s)) != HPCS_OK) return rc;
-    HPCS_CUDA(cudaMemcpyAsync(d + lo, o + lo, size_t(n - lo) * sizeof(U), cudaMemcpyDeviceToDevice, s));
+    if ((rc = enqueue_select<U, KIND>(ctx, d + lo, n - lo, rank - lo, s, &st, o + lo)) != HPCS_OK) return rc;
+    if ((rc = enqueue_partition<U, KIND>(ctx, o + lo, n - lo, st, d + lo, s)) != HPCS_OK) return rc;
     int64_t less_eq[2] = {0, 0};  // SelectState::less and ::eq are adjacent
     HPCS_CUDA(cudaMemcpyAsync(less_eq, &st->less, sizeof(less_eq), cudaMemcpyDeviceToHost, s));
     HPCS_CUDA(cudaStreamSynchronize(s));

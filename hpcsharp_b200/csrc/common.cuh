@@ -177,12 +177,13 @@ __device__ __forceinline__ uint4 ldg_stream_v4(const void* p) {
 
 // Calls f(k, nv) for the keys of keys[0..n) in groups of E = 16 / sizeof(U): k holds E keys,
 // the first nv of them valid.  The 16-byte-aligned body goes as vectors, VPT per thread in
-// flight (vector j of a round at base + j*G + global thread id, G = grid threads); the
+// flight (vector j of a round at base + j*G + global thread id, G = threads of the first `ctas` CTAs,
+// which alone make the call); the
 // unaligned head (< E keys) and the ragged tail (< E keys) go to lanes 0 and 1 of the grid's
 // first warp.  Every lane of a warp makes the same calls (nv = 0 pads), so f may use warp
 // collectives.
 template <class U, int VPT, class F>
-__device__ __forceinline__ void visit_keys(const U* __restrict__ keys, int64_t n, F&& f) {
+__device__ __forceinline__ void visit_keys(const U* __restrict__ keys, int64_t n, uint32_t ctas, F&& f) {
   constexpr int E = int(16 / sizeof(U));
   union Vec {
     uint4 v;
@@ -194,7 +195,7 @@ __device__ __forceinline__ void visit_keys(const U* __restrict__ keys, int64_t n
   const int64_t nvec = (n - head) / E;
   const int64_t rest = head + nvec * E;  // first key of the tail
   const uint4* vp = reinterpret_cast<const uint4*>(keys + head);
-  const int64_t G = int64_t(gridDim.x) * blockDim.x;
+  const int64_t G = int64_t(ctas) * blockDim.x;
   const int64_t gtid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   for (int64_t base = 0; base < nvec; base += G * VPT) {  // uniform over the grid
     Vec v[VPT];
