@@ -113,7 +113,7 @@ def device_key(ctx: "native.Context") -> dict:
 def tune(ctx: "native.Context | None" = None, total_keys: int = 24 << 20, reps: int = 5,
          log=print) -> dict:
     own = ctx is None
-    ctx = ctx or native.Context(0)
+    ctx = ctx or native.Context(0, seg_grid_min_keys=-1)  # the variants themselves, no grid level
     try:
         variants = native.seg_variants()
         bounds = class_bounds()

@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "seg_tile.cuh"
 #include "segmented.cuh"
 #include "sort_host.cuh"
 
@@ -58,8 +59,8 @@ inline bool seg_variant_fits(int v, int w_index, int c) {
 // choice on a B200 (148 SMs), recorded with its measurements in tune/b200_148sm.json.
 inline hpcs_seg_tuning seg_default_tuning() {
   hpcs_seg_tuning t{};
-  const int v4[HPCS_SEG_CLASSES] = {0, 1, 2, 5, 6, 8, 6, 8};
-  const int v8[HPCS_SEG_CLASSES] = {1, 2, 10, 6, 8, 9, 9, 9};
+  const int v4[HPCS_SEG_CLASSES] = {0, 1, 2, 5, 6, 8, 9, 8};
+  const int v8[HPCS_SEG_CLASSES] = {1, 2, 10, 6, 8, 9, 9, 8};
   for (int c = 0; c < HPCS_SEG_CLASSES; c++) {
     t.variant[0][c] = v4[c];
     t.variant[1][c] = v8[c];
@@ -96,6 +97,7 @@ inline int launch_seg_variant(hpcs_ctx* ctx, int v, bool large, const SegDesc* d
     }
     return HPCS_OK;
   };
+  constexpr int W = MODE == RANK_PEER_MASK ? 32 : 46;  // keys per thread of the wide tiles (lane masks take room)
 #define HPCS_SEG_BLOCK(NTV, KPTV)                                                                          \
   (large ? go(segmented_sort_kernel<NTV, KPTV, MODE, true>, NTV, SegSmem<NTV, KPTV, MODE>::BYTES, 1)      \
          : go(segmented_sort_kernel<NTV, KPTV, MODE, false>, NTV, SegSmem<NTV, KPTV, MODE>::BYTES, 1))
@@ -108,8 +110,12 @@ inline int launch_seg_variant(hpcs_ctx* ctx, int v, bool large, const SegDesc* d
     case 5: return HPCS_SEG_BLOCK(256, 8);
     case 6: return HPCS_SEG_BLOCK(256, 16);
     case 7: return HPCS_SEG_BLOCK(512, 8);
-    case 8: return HPCS_SEG_BLOCK(512, 16);
-    case 9: return HPCS_SEG_BLOCK(512, 32);
+    case 8:
+      return large ? go(seg_tile_kernel<512, W, MODE>, 512, SegTileSmem<512, W, MODE>::BYTES, 1)
+                   : go(segmented_sort_kernel<512, 16, MODE, false>, 512, SegSmem<512, 16, MODE>::BYTES, 1);
+    case 9:
+      return large ? go(seg_tile_kernel<256, 32, MODE>, 256, SegTileSmem<256, 32, MODE>::BYTES, 1)
+                   : go(segmented_sort_kernel<512, 32, MODE, false>, 512, SegSmem<512, 32, MODE>::BYTES, 1);
     case 10: return go(seg_warp_kernel<32, 8, MODE>, 256, WarpSegSmem<32, MODE>::BYTES, 8);
     default: return fail(HPCS_ERR_RANGE, "unknown segmented-sort variant");
   }
