@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(FIN_NT, 1) select_finish_kernel(const U* __res
                                                                  int64_t k) {
   using KO = KeyOrder<U, KIND>;
   constexpr int E = int(16 / sizeof(U));
-  extern __shared__ __align__(16) unsigned char smem[];
+  extern __shared__ __align__(128) unsigned char smem[];
   FinishSmem& sm = *reinterpret_cast<FinishSmem*>(smem);
   __shared__ uint32_t s_w[8];
   __shared__ uint32_t s_pick[3];
