@@ -230,8 +230,8 @@ __global__ void __launch_bounds__(NT, 1) lookback_pass_kernel(SortArgs args) {
     for (int i = lane; i < 2 * RADIX; i += 32) msk_w[i] = 0u;
   const uint32_t n32 = uint32_t(n);
   const Digit<U, KIND> dig(shift);
-  // When this pass's two most frequent values hold more than 3/4 of the keys, their lanes rank
-  // with one atomic per warp instruction each (ordered-atomic mode only).
+  // This pass's two most frequent values hold much of the keys: they rank by votes (ordered-atomic
+  // mode only).
   const bool grouped = MODE == RANK_ORDERED_ATOMIC && plan->grouped[pass] != 0;
   const uint32_t heavy = uint32_t(plan->heavy[pass]), heavy2 = uint32_t(plan->heavy2[pass]);
   const int sd = tid / G, sq = tid % G;  // the digit and warp group this thread scans
@@ -347,11 +347,13 @@ __global__ void __launch_bounds__(NT, 1) lookback_pass_kernel(SortArgs args) {
 #pragma unroll
     for (int i = 0; i < (KPT + 1) / 2; i++) rank[i] = 0u;
     if (grouped) {
+      FrequentRanks fr(heavy, heavy2);
 #pragma unroll
       for (int i = 0; i < KPT; i++) {
         const int idx = wbase + i * 32 + lane;
-        rank[i / 2] |= rank_in_warp_top2(cnt_w, dig(key[i]), FULL || idx < tile_n, heavy, heavy2, lane) << (16 * (i & 1));
+        rank[i / 2] |= fr.rank(cnt_w, dig(key[i]), FULL || idx < tile_n) << (16 * (i & 1));
       }
+      fr.close(cnt_w, lane);
     } else {
 #pragma unroll
       for (int i = 0; i < KPT; i++) {

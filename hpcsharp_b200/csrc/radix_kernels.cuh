@@ -47,7 +47,7 @@ struct SortPlan {
   int32_t heavy[MAX_PASSES];              // the most frequent value of each digit (lowest on ties)
   int32_t skewed[MAX_PASSES];             // 1 when that value holds more than 1/32 of the keys
   int32_t heavy2[MAX_PASSES];             // the second most frequent value
-  int32_t grouped[MAX_PASSES];            // 1 when the two hold more than 3/4 of the keys
+  int32_t grouped[MAX_PASSES];            // 1 when the first holds more than 5/16 of the keys
 };
 
 struct SortArgs {
@@ -264,7 +264,7 @@ __device__ __forceinline__ void hist_all_digits_body(const U* __restrict__ keys,
       plan->heavy[d] = d < P ? int(255u - uint32_t(s_heavy[d] & 255ull)) : 0;
       plan->skewed[d] = d < P && int64_t(s_heavy[d] >> 8) > n / 32 ? 1 : 0;
       plan->heavy2[d] = d < P && s_heavy2[d] ? int(255u - uint32_t(s_heavy2[d] & 255ull)) : plan->heavy[d];
-      plan->grouped[d] = d < P && int64_t(s_heavy[d] >> 8) + int64_t(s_heavy2[d] >> 8) > n / 4 * 3 ? 1 : 0;
+      plan->grouped[d] = d < P && int64_t(s_heavy[d] >> 8) > n / 16 * 5 ? 1 : 0;
       if (d >= P) {
         plan->src_sel[d] = -1;
         continue;
@@ -346,29 +346,35 @@ __device__ __forceinline__ uint32_t rank_in_warp(uint32_t* cnt, uint32_t* msk, u
   }
 }
 
-// Ordered-atomic ranking for a pass whose two most frequent digit values h1, h2 hold much of
-// the keys: the lanes of a warp instruction holding h1 (or h2) take one atomicAdd of their
-// count, made by the lowest of them, and rank among themselves by popcount, instead of
-// serialising on one counter; other lanes rank with their own atomic.  Same ranks as
-// rank_in_warp<RANK_ORDERED_ATOMIC>.  All lanes must call it (it uses warp votes).
-__device__ __forceinline__ uint32_t rank_in_warp_top2(uint32_t* cnt, uint32_t d, bool valid, uint32_t h1,
-                                                      uint32_t h2, int lane) {
-  const bool is1 = valid && d == h1;
-  const bool is2 = valid && d == h2 && h2 != h1;
-  const uint32_t m1 = __ballot_sync(0xFFFFFFFFu, is1);
-  const uint32_t m2 = __ballot_sync(0xFFFFFFFFu, is2);
-  const int l1 = m1 ? __ffs(m1) - 1 : 0;
-  const int l2 = m2 ? __ffs(m2) - 1 : 0;
-  uint32_t b1 = 0, b2 = 0, r = 0;
-  if (m1 && lane == l1) b1 = atomicAdd(&cnt[h1], uint32_t(__popc(m1)));
-  if (m2 && lane == l2) b2 = atomicAdd(&cnt[h2], uint32_t(__popc(m2)));
-  if (valid && !is1 && !is2) r = atomicAdd(&cnt[d], 1u);
-  b1 = __shfl_sync(0xFFFFFFFFu, b1, l1);
-  b2 = __shfl_sync(0xFFFFFFFFu, b2, l2);
-  if (is1) r = b1 + uint32_t(__popc(m1 & lanemask_lt()));
-  if (is2) r = b2 + uint32_t(__popc(m2 & lanemask_lt()));
-  return r;
-}
+// Ordered-atomic ranking for a pass whose two most frequent digit values h1, h2 hold much of the keys:
+// their lanes would serialise on two counters.  A value's keys in a warp are counted in a register
+// instead (every lane holds the same count) and rank by that count and a popcount of the vote, without
+// touching shared memory; the other lanes rank with their own atomic.  Same ranks as
+// rank_in_warp<RANK_ORDERED_ATOMIC>.  All lanes call rank() once per row of keys, then close() once.
+// The votes are worth it from h1 ~ 0.3 of the keys on, whether h2 is as frequent or rare (us per look-back
+// pass, atomics / votes, one value of share 0.25, 0.35, 0.5, 1: 32 Mi u32 keys 113 / 124, 126 / 125,
+// 141 / 123, 190 / 104; 16 Mi u64 pairs 111 / 113, 115 / 112, 123 / 111, 138 / 98; two values of together
+// 0.5, 0.7, 1: u32 keys 119 / 121, 129 / 118, 140 / 109).
+struct FrequentRanks {
+  uint32_t h1, h2;  // h2 == RADIX: there is no second value
+  uint32_t c1 = 0u, c2 = 0u;
+  __device__ __forceinline__ FrequentRanks(uint32_t a, uint32_t b) : h1(a), h2(b != a ? b : uint32_t(RADIX)) {}
+  __device__ __forceinline__ uint32_t rank(uint32_t* cnt, uint32_t d, bool valid) {
+    const bool is1 = valid && d == h1, is2 = valid && d == h2;
+    const uint32_t m1 = __ballot_sync(0xFFFFFFFFu, is1), m2 = __ballot_sync(0xFFFFFFFFu, is2);
+    uint32_t r = 0u;
+    if (valid && !is1 && !is2) r = atomicAdd(&cnt[d], 1u);
+    if (is1 || is2) r = (is1 ? c1 : c2) + uint32_t(__popc((is1 ? m1 : m2) & lanemask_lt()));
+    c1 += uint32_t(__popc(m1));
+    c2 += uint32_t(__popc(m2));
+    return r;
+  }
+  // the two counters, which no atomic touched
+  __device__ __forceinline__ void close(uint32_t* cnt, int lane) const {
+    if (lane == 0) cnt[h1] = c1;
+    if (lane == 1 && h2 < uint32_t(RADIX)) cnt[h2] = c2;
+  }
+};
 
 // Issue the bulk copy of tile t (keys, then items, at dst) with mbar as its barrier (called by one
 // thread).  The 16-byte-aligned body is copied by the TMA engine; the ragged tail (< 16 bytes) is
