@@ -67,7 +67,7 @@ int ensure_seg_streams(hpcs_ctx* ctx) {
 
 }  // namespace
 
-int seg_build_groups(const hpcs_seg_tuning& tuning, const hpcs_segment* segs, int64_t nsegs,
+int seg_build_groups(const hpcs_seg_tuning& tuning, int few_tiled, const hpcs_segment* segs, int64_t nsegs,
                      std::vector<SegDesc>& table, std::vector<SegGroup>& groups, size_t& scratch) {
   int rc = validate(segs, nsegs);
   if (rc != HPCS_OK) return rc;
@@ -80,6 +80,17 @@ int seg_build_groups(const hpcs_seg_tuning& tuning, const hpcs_segment* segs, in
     const int v = tuning.variant[w == 8 ? 1 : 0][seg_class_of(segs[i].n)];
     var[i] = 2 * v + (seg_variant_large(v, segs[i].n, w) ? 1 : 0);
     group_bytes[var[i]] += double(segs[i].n) * w;
+  }
+  // Few tiled arrays: one array's own time is what counts, and the wide shape sorts an array in about
+  // half the narrow one's.  The line: the narrow shape would hold them all at once (two CTAs per SM), so
+  // its better throughput does not come to bear (whole batches, us, narrow / wide, by tiled arrays: 7
+  // 153 / 112, 74 266 / 220, 179 359 / 232, 263 416 / 306, 292 343 / 327, 430 402 / 454, 597 523 / 609).
+  constexpr int NARROW = 2 * SEG_NARROW_TILES + 1, WIDE = 2 * SEG_WIDE_TILES + 1;
+  const bool few = std::count(var.begin(), var.end(), NARROW) + std::count(var.begin(), var.end(), WIDE) <= few_tiled;
+  if (few) {
+    std::replace(var.begin(), var.end(), NARROW, WIDE);
+    group_bytes[WIDE] += group_bytes[NARROW];
+    group_bytes[NARROW] = 0.0;
   }
   // groups in decreasing total bytes (the heaviest is launched first, on the caller's
   // stream), arrays within a group largest first
@@ -103,7 +114,7 @@ int seg_build_groups(const hpcs_seg_tuning& tuning, const hpcs_segment* segs, in
     const int v = gid / 2;
     const bool large = (gid & 1) != 0;
     if (groups.empty() || 2 * groups.back().variant + (groups.back().large ? 1 : 0) != gid)
-      groups.push_back({v, large, int(j), 0});
+      groups.push_back({v, large, int(j), 0, few && gid == WIDE ? sg.n * key_bytes(sg.dtype) : 0});
     groups.back().count++;
     SegDesc& d = table[j];
     d.keys = sg.keys;
@@ -140,7 +151,7 @@ int launch_groups_mode(hpcs_ctx* ctx, const SegDesc* d_desc, const std::vector<S
   for (int g = 0; g < ng; g++) {
     cudaStream_t st = g == 0 ? s : ctx->seg_streams[(g - 1) % hpcs_ctx::SEG_BRANCHES];
     if ((rc = launch_seg_variant<MODE>(ctx, groups[g].variant, groups[g].large, d_desc + groups[g].first,
-                                       groups[g].count, d_queues + g, st)) != HPCS_OK)
+                                       groups[g].count, d_queues + g, st, groups[g].longest)) != HPCS_OK)
       return rc;
   }
   for (int b = 0; b < hpcs_ctx::SEG_BRANCHES && b < ng - 1; b++) {
@@ -367,7 +378,7 @@ int hpcs_sort_segmented_dev(hpcs_ctx* ctx, const hpcs_segment* segs, int64_t nse
   std::vector<SegDesc> table;
   std::vector<SegGroup> groups;
   size_t scratch = 0;
-  if ((rc = seg_build_groups(ctx->seg_tuning, rest.data(), int64_t(rest.size()), table, groups, scratch)) != HPCS_OK)
+  if ((rc = seg_build_groups(ctx->seg_tuning, seg_few_tiled(ctx), rest.data(), int64_t(rest.size()), table, groups, scratch)) != HPCS_OK)
     return rc;
   SegGrid grid;
   if ((rc = seg_grid_build(segs, grid_idx, ctx->rank_mode, ctx->cfg.skip_trivial_passes,
@@ -412,7 +423,7 @@ int hpcs_segplan_create(hpcs_ctx* ctx, const hpcs_segment* segs, int64_t nsegs, 
   std::vector<SegDesc> table;
   std::vector<SegGroup> groups;
   size_t scratch = 0;
-  if ((rc = seg_build_groups(ctx->seg_tuning, rest.data(), int64_t(rest.size()), table, groups, scratch)) != HPCS_OK)
+  if ((rc = seg_build_groups(ctx->seg_tuning, seg_few_tiled(ctx), rest.data(), int64_t(rest.size()), table, groups, scratch)) != HPCS_OK)
     return rc;
   SegGrid grid;
   if ((rc = seg_grid_build(segs, grid_idx, ctx->rank_mode, ctx->cfg.skip_trivial_passes,
@@ -543,6 +554,7 @@ int hpcs_ctx_set_seg_tuning(hpcs_ctx* ctx, const hpcs_seg_tuning* t) {
       if (!seg_variant_fits(t->variant[w][c], w, c))
         return fail(HPCS_ERR_RANGE, "segmented-sort variant unknown or too small for its length class");
   ctx->seg_tuning = *t;
+  ctx->seg_tuning_set = true;
   return HPCS_OK;
 }
 

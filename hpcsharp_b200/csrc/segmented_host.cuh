@@ -34,6 +34,8 @@ constexpr SegVariant SEG_VARIANTS[] = {
     {0, 256, 4, 8}, {0, 256, 8, 8}, {0, 256, 16, 8}, {0, 256, 8, 4}, {0, 256, 16, 4},
     {1, 256, 8, 8}, {1, 256, 16, 8}, {1, 512, 8, 8}, {1, 512, 16, 8}, {1, 512, 32, 8}, {0, 256, 32, 8},
 };
+// The variants whose tiled path is seg_tile_kernel, one and two CTAs per SM.
+constexpr int SEG_WIDE_TILES = 8, SEG_NARROW_TILES = 9;
 constexpr int SEG_NVARIANTS = int(sizeof(SEG_VARIANTS) / sizeof(SEG_VARIANTS[0]));
 
 // Longest array a variant sorts for a key width (-1: any, block level with scratch beyond a tile).
@@ -78,12 +80,19 @@ inline int seg_setup_kernel(Kernel k, int nt, size_t smem, int& blocks) {
 }
 
 // One persistent launch of variant v over `nsegs` descriptors (its queue already zeroed);
-// `large` selects the block level's tiled path (arrays longer than the variant's tile).
+// `large` selects the block level's tiled path (arrays longer than the variant's tile); `longest`, where
+// not 0, the bytes of the longest array of a group in which one array's own time counts.
 template <int MODE>
 inline int launch_seg_variant(hpcs_ctx* ctx, int v, bool large, const SegDesc* d_desc, int nsegs,
-                              uint32_t* d_queue, cudaStream_t s) {
-  static int blocks_by_dev[64][SEG_NVARIANTS][2] = {};
-  int& blocks = blocks_by_dev[ctx->device & 63][v][large ? 1 : 0];
+                              uint32_t* d_queue, cudaStream_t s, int64_t longest = 0) {
+  constexpr int W = MODE == RANK_PEER_MASK ? 32 : 46;  // keys per thread of the wide tiles (lane masks take room)
+  // A short tile takes about a whole one's time: the wide shape's tile is the one whose whole tiles hold
+  // the longest array in the fewest rows (u64 arrays of up to 12 Ki keys in a batch: 162 us in two tiles
+  // of 46 4-byte rows).
+  auto rows = [&](int kpt) { return (longest + 512 * 4 * kpt - 1) / (512 * 4 * kpt) * kpt; };
+  const bool short_tiles = v == SEG_WIDE_TILES && large && longest > 0 && rows(32) < rows(W);
+  static int blocks_by_dev[64][SEG_NVARIANTS][3] = {};
+  int& blocks = blocks_by_dev[ctx->device & 63][v][short_tiles ? 2 : large ? 1 : 0];
   SegParams prm{d_desc, nsegs, d_queue, device_error_word(ctx), uint64_t(ctx->cfg.spin_limit_ns)};
   auto go = [&](auto k, int nt, size_t smem, int per_block) -> int {
     int rc = seg_setup_kernel(k, nt, smem, blocks);
@@ -97,7 +106,6 @@ inline int launch_seg_variant(hpcs_ctx* ctx, int v, bool large, const SegDesc* d
     }
     return HPCS_OK;
   };
-  constexpr int W = MODE == RANK_PEER_MASK ? 32 : 46;  // keys per thread of the wide tiles (lane masks take room)
 #define HPCS_SEG_BLOCK(NTV, KPTV)                                                                          \
   (large ? go(segmented_sort_kernel<NTV, KPTV, MODE, true>, NTV, SegSmem<NTV, KPTV, MODE>::BYTES, 1)      \
          : go(segmented_sort_kernel<NTV, KPTV, MODE, false>, NTV, SegSmem<NTV, KPTV, MODE>::BYTES, 1))
@@ -111,6 +119,7 @@ inline int launch_seg_variant(hpcs_ctx* ctx, int v, bool large, const SegDesc* d
     case 6: return HPCS_SEG_BLOCK(256, 16);
     case 7: return HPCS_SEG_BLOCK(512, 8);
     case 8:
+      if (short_tiles) return go(seg_tile_kernel<512, 32, MODE>, 512, SegTileSmem<512, 32, MODE>::BYTES, 1);
       return large ? go(seg_tile_kernel<512, W, MODE>, 512, SegTileSmem<512, W, MODE>::BYTES, 1)
                    : go(segmented_sort_kernel<512, 16, MODE, false>, 512, SegSmem<512, 16, MODE>::BYTES, 1);
     case 9:
@@ -129,6 +138,7 @@ struct SegGroup {
   bool large;
   int first;
   int count;
+  int64_t longest;  // bytes of its longest array where one array's own time counts, else 0
 };
 
 // Whether variant v sorts an array of n keys of width w with its tiled (scratch) path.
@@ -139,7 +149,11 @@ inline bool seg_variant_large(int v, int64_t n, int key_bytes) {
 // Orders the descriptors by (variant, bytes descending), fills `groups`, and returns through
 // `scratch` the bytes of scratch the block-level arrays longer than one tile need (their
 // scratch fields hold offsets until seg_relocate).
-int seg_build_groups(const hpcs_seg_tuning& tuning, const hpcs_segment* segs, int64_t nsegs,
+// The arrays of the narrow tiled shape up to which a batch runs them in the wide one: what the narrow
+// shape holds at once.  A table set by the caller is followed as it is (-1).
+inline int seg_few_tiled(const hpcs_ctx* ctx) { return ctx->seg_tuning_set ? -1 : 2 * ctx->sms; }
+// Up to `few_tiled` arrays of the narrow tiled shape run in the wide one (negative: the table as it is).
+int seg_build_groups(const hpcs_seg_tuning& tuning, int few_tiled, const hpcs_segment* segs, int64_t nsegs,
                      std::vector<SegDesc>& table, std::vector<SegGroup>& groups, size_t& scratch);
 void seg_relocate(std::vector<SegDesc>& table, const std::vector<SegGroup>& groups, void* base);
 

@@ -71,6 +71,7 @@ struct hpcs_ctx {
   // batched segmented sort: variant per (key width, length class), and the helper streams
   // and events that run the launches of different variants concurrently
   hpcs_seg_tuning seg_tuning{};
+  bool seg_tuning_set = false;  // by the caller: followed as it is
   static constexpr int SEG_BRANCHES = 3;
   cudaStream_t seg_streams[SEG_BRANCHES] = {};
   cudaEvent_t seg_fork = nullptr;

@@ -249,7 +249,8 @@ int hpcs_segplan_destroy(hpcs_segplan* plan);
  * in registers and shared memory) or a block-level one (one CTA per array, in shared memory
  * when the array fits one tile, else tile by tile with scratch).  A context starts with the
  * built-in table, chosen on a B200 by the project's autotuner (hpcsharp_b200/autotune.py);
- * hpcs_ctx_set_seg_tuning replaces it.  A plan uses the table in force when it is created.
+ * hpcs_ctx_set_seg_tuning replaces it.  With the built-in table a batch of few tiled arrays (at
+ * most two per SM) takes the wide tiled shape for them.  A plan uses the table in force when it is created.
  * Arrays of one variant go to one persistent launch; the launches of different variants run
  * concurrently on forked streams (inside the plan's graph, as graph branches). */
 #define HPCS_SEG_CLASSES 8
