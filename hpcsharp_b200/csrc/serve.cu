@@ -327,6 +327,13 @@ void launch_batch(hpcs_server* sv) {
     d.scratch = coalesced_needs_scratch(c->seg_tuning, q->r) ? keys + up256(size_t(q->r.n) * w) : nullptr;
     cudaMemcpyAsync(keys, q->r.input, size_t(q->r.n) * w, cudaMemcpyHostToDevice, s);
   }
+  // few tiled arrays take the wide tiled shape, as in a batched sort
+  for (SegGroup& g : groups) {
+    if (g.variant != SEG_NARROW_TILES || !g.large || g.count > seg_few_tiled(c)) continue;
+    const SegDesc& longest = sv->host_table[g.first];
+    g.variant = SEG_WIDE_TILES;
+    g.longest = longest.n * dtype_bytes(longest.dtype);
+  }
   cudaMemcpyAsync(d_table, sv->host_table, n * sizeof(SegDesc), cudaMemcpyHostToDevice, s);
   c->last_stream = s;
   int rc = seg_launch_groups(c, d_table, groups, d_queues, s);
