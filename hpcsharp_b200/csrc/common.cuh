@@ -86,6 +86,9 @@ struct Digit<uint64_t, KIND> {
 // chain_wait returns once the predecessor has completed and its writes are visible (at once in a
 // plain launch); every chained kernel calls it before it touches memory or exits.  chain_release
 // lets the successor's CTAs be scheduled as this grid's finish.
+// The wait orders a kernel's loads only if the compiler may not take them for loads of memory that
+// nothing writes during the kernel: a chained kernel has no __restrict__ pointer (a "memory" clobber
+// does not hold back loads through one) and makes no __ldg or other non-coherent load.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -175,6 +178,17 @@ __device__ __forceinline__ uint4 ldg_stream_v4(const void* p) {
   return v;
 }
 
+// The same without the read-only promise: for what a chained predecessor may have written, ordered
+// behind chain_wait by the "memory" clobber.
+__device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+
 // Calls f(k, nv) for the keys of keys[0..n) in groups of E = 16 / sizeof(U): k holds E keys,
 // the first nv of them valid.  The 16-byte-aligned body goes as vectors, VPT per thread in
 // flight (vector j of a round at base + j*G + global thread id, G = threads of the first `ctas` CTAs,
@@ -183,7 +197,7 @@ __device__ __forceinline__ uint4 ldg_stream_v4(const void* p) {
 // first warp.  Every lane of a warp makes the same calls (nv = 0 pads), so f may use warp
 // collectives.
 template <class U, int VPT, class F>
-__device__ __forceinline__ void visit_keys(const U* __restrict__ keys, int64_t n, uint32_t ctas, F&& f) {
+__device__ __forceinline__ void visit_keys(const U* keys, int64_t n, uint32_t ctas, F&& f) {
   constexpr int E = int(16 / sizeof(U));
   union Vec {
     uint4 v;
@@ -202,7 +216,7 @@ __device__ __forceinline__ void visit_keys(const U* __restrict__ keys, int64_t n
 #pragma unroll
     for (int j = 0; j < VPT; j++) {
       const int64_t idx = base + j * G + gtid;
-      v[j].v = idx < nvec ? __ldg(vp + idx) : make_uint4(0u, 0u, 0u, 0u);
+      v[j].v = idx < nvec ? ld_stream_v4(vp + idx) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int j = 0; j < VPT; j++) f(v[j].k, base + j * G + gtid < nvec ? E : 0);
@@ -226,7 +240,7 @@ __device__ __forceinline__ void visit_keys(const U* __restrict__ keys, int64_t n
 // Appends the keys k[e] whose bit e of `take` is set to dst at a position drawn from *counter
 // (one atomic per warp); positions at or beyond `cap` are not written.  All lanes call it.
 template <class U, int E>
-__device__ __forceinline__ void warp_append(const U* k, uint32_t take, U* __restrict__ dst,
+__device__ __forceinline__ void warp_append(const U* k, uint32_t take, U* dst,
                                             unsigned long long* counter, int64_t cap) {
   const int lane = threadIdx.x & 31;
   const uint32_t c = __popc(take);

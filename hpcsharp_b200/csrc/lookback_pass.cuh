@@ -192,10 +192,10 @@ __global__ void __launch_bounds__(NT, 1) lookback_pass_kernel(SortArgs args) {
   volatile int* s_tile = reinterpret_cast<volatile int*>(smem + L::OFF_TILE);
   uint64_t* s_mbar = reinterpret_cast<uint64_t*>(smem + L::OFF_MBAR);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const U* __restrict__ kin = static_cast<const U*>(sel ? args.keys_b : args.keys_a);
-  U* __restrict__ kout = static_cast<U*>(sel ? args.keys_a : args.keys_b);
-  const uint32_t* __restrict__ vin = static_cast<const uint32_t*>(sel ? args.vals_b : args.vals_a);
-  uint32_t* __restrict__ vout = static_cast<uint32_t*>(sel ? args.vals_a : args.vals_b);
+  const U* kin = static_cast<const U*>(sel ? args.keys_b : args.keys_a);
+  U* kout = static_cast<U*>(sel ? args.keys_a : args.keys_b);
+  const uint32_t* vin = static_cast<const uint32_t*>(sel ? args.vals_b : args.vals_a);
+  uint32_t* vout = static_cast<uint32_t*>(sel ? args.vals_a : args.vals_b);
 
   // tickets: a grid of one CTA has one tile and needs no scanner
   const int first = gridDim.x > 1 ? 1 : 0;

@@ -62,7 +62,7 @@ template <class U, int E, int CAP>
 struct WarpStage {
   U* buf;
   uint32_t count;
-  U* __restrict__ dst;
+  U* dst;
   unsigned long long* counter;
   int64_t cap;
 
@@ -108,8 +108,8 @@ struct WarpStage {
 // grid can be large enough for all keys.  (Separate decide, histogram and pick launches took ~55 us
 // of a 285 us top-k call.)
 template <class U, int KIND>
-__global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_level_kernel(const U* __restrict__ keys, int64_t n,
-                                                                              const U* __restrict__ cand, int64_t rank,
+__global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_level_kernel(const U* keys, int64_t n,
+                                                                              const U* cand, int64_t rank,
                                                                               SelectState* st, int shift, int open_top,
                                                                               int only_full) {
   using KO = KeyOrder<U, KIND>;
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_level_kernel(c
   const bool first = shift == TOP_SHIFT;
   const bool among = first ? below <= rank && rank < below + c : true;  // rank among the candidates
   if (only_full && among) return;
-  const U* __restrict__ src = among ? cand : keys;
+  const U* src = among ? cand : keys;
   const int64_t m = among ? c : n;
   const int64_t per_cta = int64_t(SEL_NT) * SEL_VPT * E;
   const int64_t want = (m + per_cta - 1) / per_cta;
@@ -204,9 +204,9 @@ __global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_level_kernel(c
 // (top-k): the keys above that bin, all among the k largest, go to out[0..) through
 // st->gathered at once (fewer than k of them: the selected rank lies in the bin).
 template <class U, int KIND>
-__global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_compact_kernel(const U* __restrict__ keys, int64_t n,
-                                                                U* __restrict__ cand, SelectState* st,
-                                                                U* __restrict__ out, int64_t k_out) {
+__global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_compact_kernel(const U* keys, int64_t n,
+                                                                U* cand, SelectState* st,
+                                                                U* out, int64_t k_out) {
   using KO = KeyOrder<U, KIND>;
   constexpr int E = int(16 / sizeof(U));
   constexpr int CAP = 1024 / int(sizeof(U));  // 1 KiB per warp and buffer
@@ -250,8 +250,8 @@ struct FinishSmem {
 };
 
 template <class U, int KIND>
-__global__ void __launch_bounds__(FIN_NT, 1) select_finish_kernel(const U* __restrict__ cand, int64_t n, int64_t rank,
-                                                                 SelectState* st, int open_top, U* __restrict__ out,
+__global__ void __launch_bounds__(FIN_NT, 1) select_finish_kernel(const U* cand, int64_t n, int64_t rank,
+                                                                 SelectState* st, int open_top, U* out,
                                                                  int64_t k) {
   using KO = KeyOrder<U, KIND>;
   constexpr int E = int(16 / sizeof(U));
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(FIN_NT, 1) select_finish_kernel(const U* __res
     for (int j = 0; j < V; j++) {
       const int64_t at = (int64_t(j) * ctas * FIN_NT + gtid) * E;
       if (at + E <= c) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(cand + at));
+        const uint4 v = ld_stream_v4(cand + at);
 #pragma unroll
         for (int e = 0; e < E; e++) keep[j * E + e] = KO::to_ordered(reinterpret_cast<const U*>(&v)[e]);
         valid |= ((1u << E) - 1u) << (j * E);
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(512) select_gather_kernel(const U* __restrict_
 // highest) by two MSD radix selects side by side; per level a histogram of the samples matching each
 // prefix and a scan of its 256 bins by 8 warps.
 template <class U>
-__global__ void __launch_bounds__(SAMPLE_NT) select_sample_kernel(const U* __restrict__ samp, int64_t rlo, int64_t rhi,
+__global__ void __launch_bounds__(SAMPLE_NT) select_sample_kernel(const U* samp, int64_t rlo, int64_t rhi,
                                                                  SelectState* st) {
   constexpr int S = select_sample_size<U>();
   constexpr int PER = S / SAMPLE_NT;
@@ -533,9 +533,9 @@ struct WinTile {
 // Short-lived CTAs read faster than persistent ones (2^28 u32 keys, 199 us as a persistent kernel
 // that staged kept keys per warp, 5.4 TB/s; a bare read takes 150).
 template <class U, int KIND, bool COPY, bool TILES>
-__global__ void __launch_bounds__(WIN_NT, TILES || sizeof(U) == 8 ? 3 : 4) select_window_kernel(const U* __restrict__ keys, int64_t n,
-                                                               U* __restrict__ cand, SelectState* st,
-                                                               U* __restrict__ copy, WinTile* __restrict__ tiles,
+__global__ void __launch_bounds__(WIN_NT, TILES || sizeof(U) == 8 ? 3 : 4) select_window_kernel(const U* keys, int64_t n,
+                                                               U* cand, SelectState* st,
+                                                               U* copy, WinTile* tiles,
                                                                int steps) {
   using KO = KeyOrder<U, KIND>;
   constexpr int E = int(16 / sizeof(U)), V = 4, T = win_tile<U>(), NW = WIN_NT / 32;
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(WIN_NT, TILES || sizeof(U) == 8 ? 3 : 4) selec
     if (aligned && tn == T) {  // uniform over the CTA
       const uint4* p = reinterpret_cast<const uint4*>(keys + t0);
 #pragma unroll
-      for (int j = 0; j < V; j++) r[j].v = ldg_stream_v4(p + j * WIN_NT + tid);
+      for (int j = 0; j < V; j++) r[j].v = ld_stream_v4(p + j * WIN_NT + tid);
       if (COPY) {
         uint4* q = reinterpret_cast<uint4*>(copy + t0);
 #pragma unroll
@@ -677,10 +677,10 @@ __device__ __forceinline__ int part_class(U k, U v_ordered) {
 // A warp per tile: counts[tile] = {keys < v, keys == v}, from the keys below the window and the tile's
 // candidates (a few percent of the keys), or from the keys themselves when the window missed.
 template <class U, int KIND>
-__global__ void __launch_bounds__(256) partition_count_kernel(const U* __restrict__ keys, int64_t n,
-                                                              const U* __restrict__ cand, const SelectState* st,
-                                                              const WinTile* __restrict__ tiles, int64_t ntiles,
-                                                              uint2* __restrict__ counts) {
+__global__ void __launch_bounds__(256) partition_count_kernel(const U* keys, int64_t n,
+                                                              const U* cand, const SelectState* st,
+                                                              const WinTile* tiles, int64_t ntiles,
+                                                              uint2* counts) {
   constexpr int T = win_tile<U>();
   chain_wait();
   chain_release();
@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(256) partition_count_kernel(const U* __restric
 }
 
 // One CTA: counts[] into exclusive starts, each thread a run of consecutive tiles.
-static __global__ void __launch_bounds__(1024) partition_scan_kernel(uint2* __restrict__ counts, int64_t ntiles) {
+static __global__ void __launch_bounds__(1024) partition_scan_kernel(uint2* counts, int64_t ntiles) {
   __shared__ uint32_t s_w[2][32];
   chain_wait();
   chain_release();
@@ -749,10 +749,10 @@ static __global__ void __launch_bounds__(1024) partition_scan_kernel(uint2* __re
 // keys in class order in shared memory first took more instructions than the fewer sectors saved: 33 M
 // f32 keys 70 us.)
 template <class U, int KIND>
-__global__ void __launch_bounds__(PART_NT, 3) partition_scatter_kernel(const U* __restrict__ keys, int64_t n,
+__global__ void __launch_bounds__(PART_NT, 3) partition_scatter_kernel(const U* keys, int64_t n,
                                                                     const SelectState* st,
-                                                                    const uint2* __restrict__ starts,
-                                                                    U* __restrict__ out) {
+                                                                    const uint2* starts,
+                                                                    U* out) {
   constexpr int T = win_tile<U>(), KPT = T / PART_NT, SUB = 32 * KPT, NW = PART_NT / 32;
   __shared__ uint32_t s_c[2][NW];
   chain_wait();
@@ -819,8 +819,8 @@ __global__ void __launch_bounds__(PART_NT, 3) partition_scatter_kernel(const U* 
 // The keys above the level-0 bin are already in out (select_compact_kernel); this appends the
 // candidates > v (the level-0 bin's keys) and fills the rest with copies of v.
 template <class U, int KIND>
-__global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) topk_gather_kernel(const U* __restrict__ cand, int64_t k,
-                                                             SelectState* st, U* __restrict__ out) {
+__global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) topk_gather_kernel(const U* cand, int64_t k,
+                                                             SelectState* st, U* out) {
   using KO = KeyOrder<U, KIND>;
   constexpr int E = int(16 / sizeof(U));
   chain_wait();
@@ -855,7 +855,7 @@ __host__ __device__ constexpr int topk_small_sort_max() {
 constexpr int TOPK_SMALL_SORT_NT = 128;
 
 template <class U, int KIND>
-__global__ void __launch_bounds__(TOPK_SMALL_SORT_NT) topk_small_sort_kernel(U* __restrict__ out, int k) {
+__global__ void __launch_bounds__(TOPK_SMALL_SORT_NT) topk_small_sort_kernel(U* out, int k) {
   using KO = KeyOrder<U, KIND>;
   __shared__ U s[topk_small_sort_max<U>()];
   chain_wait();
