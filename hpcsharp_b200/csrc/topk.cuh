@@ -42,11 +42,18 @@ struct SelectState {
   uint64_t threshold;           // the window's lower end
   uint64_t threshold_hi;        // the window's upper end (inclusive)
   unsigned long long below;     // keys below the window
-  int32_t mode;        // SEL_MODE_CAND (select among the candidates) or SEL_MODE_FULL
+  int32_t mode;        // where the levels look (SelMode)
   uint32_t ticket;     // CTAs of the current level that are through
   uint32_t hist[256];
 };
-enum : int32_t { SEL_MODE_FULL = 0, SEL_MODE_CAND = 1 };
+// Where the levels look: the window's candidates (CAND), the candidates of the top-byte bin that level 0
+// chose among all keys (FULL), those strictly between the window's ends (INSIDE), or nowhere, since the
+// selected key is one of the ends (DONE).  All but CAND are the shift of the first level that the finish runs.
+template <class U>
+struct SelMode {
+  static constexpr int32_t TOP = int32_t(sizeof(U) * 8) - 8;
+  static constexpr int32_t CAND = 255, FULL = TOP - 8, INSIDE = TOP, DONE = -1;
+};
 
 constexpr int SEL_NT = 512;
 constexpr int SEL_COPIES = 32;
@@ -107,11 +114,17 @@ struct WarpStage {
 // rank must fall among the candidates.  CTAs beyond what the keys can use return at once, so the
 // grid can be large enough for all keys.  (Separate decide, histogram and pick launches took ~55 us
 // of a 285 us top-k call.)
-template <class U, int KIND>
+// FINISH: select_finish_kernel takes the candidates, so level 0 has work only where the rank is not
+// among them, or where they are more than `limit`.  So many more than expected are copies of the window's
+// ends (a value between them that filled as much would have filled the sample too): level 0 counts the
+// copies, and the rank falls on an end (DONE) or strictly between, where the expected few keys lie
+// (INSIDE: compacted anew).  The cluster of the finish would read them all once per level: the 1000
+// largest of 2^27 u32 keys, half of them the largest value, 2590 -> 467 us, all keys equal 4950 -> 743.
+template <class U, int KIND, bool FINISH>
 __global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_level_kernel(const U* keys, int64_t n,
                                                                               const U* cand, int64_t rank,
                                                                               SelectState* st, int shift, int open_top,
-                                                                              int only_full) {
+                                                                              int64_t limit) {
   using KO = KeyOrder<U, KIND>;
   constexpr int E = int(16 / sizeof(U));
   constexpr int TOP_SHIFT = int(sizeof(U) * 8) - 8;
@@ -127,23 +140,48 @@ __global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_level_kernel(c
   const int64_t c = st->cand_count, below = open_top ? n - c : int64_t(st->below);
   const bool first = shift == TOP_SHIFT;
   const bool among = first ? below <= rank && rank < below + c : true;  // rank among the candidates
-  if (only_full && among) return;
+  bool wide = false;
+  if (FINISH && among) {
+    if (c <= limit) return;
+    wide = st->threshold != st->threshold_hi;  // (equal ends: the finish reads no candidate)
+    if (!wide) return;
+  }
   const U* src = among ? cand : keys;
   const int64_t m = among ? c : n;
   const int64_t per_cta = int64_t(SEL_NT) * SEL_VPT * E;
-  const int64_t want = (m + per_cta - 1) / per_cta;
+  // (the whole grid where the last CTA resets cand_count: no CTA may read it after that)
+  const int64_t want = ((wide ? n : m) + per_cta - 1) / per_cta;
   const uint32_t active = want < 1 ? 1u : (want < int64_t(gridDim.x) ? uint32_t(want) : gridDim.x);
   if (blockIdx.x >= active) return;
   const U prefix = first ? U(0) : U(st->prefix), mask = first ? U(0) : U(st->mask);
   for (int i = tid; i < 256 * SEL_COPIES; i += SEL_NT) sh[i] = 0;
   __syncthreads();
-  visit_keys<U, SEL_VPT>(src, m, active, [&](const U* k, int nv) {
+  if (FINISH && wide) {  // bins 0 and 1: the copies of the window's ends
+    const U lo = U(st->threshold), hi = U(st->threshold_hi);
+    uint32_t nlo = 0u, nhi = 0u;
+    visit_keys<U, SEL_VPT>(src, m, active, [&](const U* k, int nv) {
 #pragma unroll
-    for (int e = 0; e < E; e++) {
-      const U o = KO::to_ordered(k[e]);
-      if (e < nv && (o & mask) == prefix) atomicAdd(&sh[((uint32_t(o >> shift) & 0xFFu) * SEL_COPIES) + lane], 1u);
+      for (int e = 0; e < E; e++) {
+        const U o = KO::to_ordered(k[e]);
+        nlo += e < nv && o == lo ? 1u : 0u;
+        nhi += e < nv && o == hi ? 1u : 0u;
+      }
+    });
+    nlo = __reduce_add_sync(0xFFFFFFFFu, nlo);
+    nhi = __reduce_add_sync(0xFFFFFFFFu, nhi);
+    if (lane == 0) {
+      atomicAdd(&sh[0], nlo);
+      atomicAdd(&sh[SEL_COPIES], nhi);
     }
-  });
+  } else {
+    visit_keys<U, SEL_VPT>(src, m, active, [&](const U* k, int nv) {
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        const U o = KO::to_ordered(k[e]);
+        if (e < nv && (o & mask) == prefix) atomicAdd(&sh[((uint32_t(o >> shift) & 0xFFu) * SEL_COPIES) + lane], 1u);
+      }
+    });
+  }
   __syncthreads();
   for (int b = tid; b < 256; b += SEL_NT) {
     uint32_t h = 0;
@@ -157,6 +195,25 @@ __global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_level_kernel(c
   if (!s_last) return;
   __threadfence();
 
+  if (FINISH && wide) {
+    if (tid == 0) {
+      const U lo = U(st->threshold), hi = U(st->threshold_hi);
+      const int64_t nlo = ld_volatile(&st->hist[0]), nhi = ld_volatile(&st->hist[1]);
+      const int64_t r = rank - below;
+      const bool at_lo = r < nlo, at_hi = !at_lo && r >= c - nhi;
+      st->mode = at_lo || at_hi ? SelMode<U>::DONE : SelMode<U>::INSIDE;
+      st->less = below + (at_lo ? 0 : at_hi ? c - nhi : nlo);
+      st->eq = at_lo ? nlo : at_hi ? nhi : 0;
+      st->rank = at_lo ? r : at_hi ? r - (c - nhi) : r - nlo;
+      st->prefix = at_lo ? uint64_t(lo) : at_hi ? uint64_t(hi) : 0ull;
+      st->mask = at_lo || at_hi ? uint64_t(U(~U(0))) : 0ull;
+      st->cand_count = 0;  // INSIDE: rebuilt by the compaction
+      st->hist[0] = 0;
+      st->hist[1] = 0;
+      st->ticket = 0;
+    }
+    return;
+  }
   // the last CTA: a scan of the 256 counts, the thread whose bin spans the rank records it
   const int64_t r = first ? (among ? rank - below : rank) : st->rank;
   const int64_t h = tid < 256 ? int64_t(ld_volatile(&st->hist[tid])) : 0;
@@ -187,7 +244,7 @@ __global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_level_kernel(c
   if (tid == 0) {
     st->ticket = 0;
     if (first) {
-      st->mode = among ? SEL_MODE_CAND : SEL_MODE_FULL;
+      st->mode = among ? SelMode<U>::CAND : SelMode<U>::FULL;
       st->less = among ? below : 0;
       if (!among) st->cand_count = 0;  // rebuilt by the compaction
     }
@@ -199,10 +256,10 @@ __global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_level_kernel(c
   }
 }
 
-// All keys were selected among: copies those whose ordered top byte matches the level-0 prefix into
-// `cand`.  With `out`
-// (top-k): the keys above that bin, all among the k largest, go to out[0..) through
-// st->gathered at once (fewer than k of them: the selected rank lies in the bin).
+// Level 0 looked beyond the candidates: copies the keys of its choice (the bin of the ordered top byte, or
+// the keys strictly between the window's ends) into `cand`.  With `out` (top-k): the keys above those, all
+// among the k largest, go to out[0..) through st->gathered at once (fewer than k of them: the selected
+// rank lies below them).
 template <class U, int KIND>
 __global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_compact_kernel(const U* keys, int64_t n,
                                                                 U* cand, SelectState* st,
@@ -213,9 +270,15 @@ __global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_compact_kernel
   __shared__ U s_buf[2][SEL_NT / 32][CAP];
   chain_wait();
   chain_release();
-  if (st->mode != SEL_MODE_FULL) return;  // the rank lies among the candidates
+  const int32_t mode = st->mode;
+  if (mode == SelMode<U>::CAND) return;  // the rank lies among the candidates
+  // DONE: only the keys above the selected one are wanted
+  if (mode == SelMode<U>::DONE && (!out || st->less + st->eq == n)) return;
   const int warp = threadIdx.x >> 5;
-  const U prefix = U(st->prefix), mask = U(st->mask);
+  // [first, last]: the keys for `cand`; none when DONE (first above last: some key lies above last)
+  const U prefix = U(st->prefix);
+  const U first = mode == SelMode<U>::FULL ? prefix : U((mode == SelMode<U>::INSIDE ? U(st->threshold) : prefix) + 1);
+  const U last = mode == SelMode<U>::FULL ? U(prefix | U(~U(st->mask))) : mode == SelMode<U>::INSIDE ? U(U(st->threshold_hi) - 1) : prefix;
   WarpStage<U, E, CAP> to_cand{s_buf[0][warp], 0u, cand, reinterpret_cast<unsigned long long*>(&st->cand_count),
                                INT64_MAX};
   WarpStage<U, E, CAP> to_out{s_buf[1][warp], 0u, out, &st->gathered, k_out};
@@ -223,9 +286,9 @@ __global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_compact_kernel
     uint32_t take = 0u, above = 0u;
 #pragma unroll
     for (int e = 0; e < E; e++) {
-      const U top = KO::to_ordered(k[e]) & mask;
-      if (e < nv && top == prefix) take |= 1u << e;
-      if (e < nv && top > prefix) above |= 1u << e;
+      const U o = KO::to_ordered(k[e]);
+      if (e < nv && o >= first && o <= last) take |= 1u << e;
+      if (e < nv && o > last) above |= 1u << e;
     }
     to_cand.add(k, take);
     if (out) to_out.add(k, above);
@@ -235,7 +298,8 @@ __global__ void __launch_bounds__(SEL_NT, SEL_CTAS_PER_SM) select_compact_kernel
 }
 
 // The remaining levels in one cluster of CTAs, for up to half a million candidates: all but those
-// that the window's two ends share or, when level 0 ran over all keys, the levels below it.  Up to 16
+// that the window's two ends share or, when level 0 ran over all keys, the levels below it (none when
+// level 0 found the selected key).  Up to 16
 // 32-bit candidates per thread stay in registers from level to level.  Per level every CTA
 // histograms its share, the 256 totals go to every CTA (distributed shared memory), one cluster
 // barrier, and every CTA picks the bin for itself.  With `out` (the k largest): then the candidates
@@ -265,14 +329,14 @@ __global__ void __launch_bounds__(FIN_NT, 1) select_finish_kernel(const U* cand,
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t ctas = gridDim.x, cta = blockIdx.x;  // the grid is one cluster
   const int64_t c = st->cand_count;
-  const bool full = st->mode == SEL_MODE_FULL;
+  const bool window = st->mode == SelMode<U>::CAND;
   const int64_t below = open_top ? n - c : int64_t(st->below);
-  U prefix = full ? U(st->prefix) : U(0), mask = full ? U(st->mask) : U(0);
-  uint32_t r = uint32_t(full ? st->rank : rank - below);
-  int64_t less = full ? st->less : below;
-  uint32_t eq = 0;
-  int shift = int(sizeof(U) * 8) - (full ? 16 : 8);
-  if (!full) {  // the digits that lo and hi share are every candidate's
+  U prefix = window ? U(0) : U(st->prefix), mask = window ? U(0) : U(st->mask);
+  uint32_t r = uint32_t(window ? rank - below : st->rank);
+  int64_t less = window ? below : st->less;
+  uint32_t eq = uint32_t(st->eq);  // (0 unless DONE)
+  int shift = window ? int(sizeof(U) * 8) - 8 : st->mode;
+  if (window) {  // the digits that lo and hi share are every candidate's
     const U lo = U(st->threshold), hi = U(st->threshold_hi);
     while (shift >= 0 && (lo >> shift) == (hi >> shift)) {
       prefix = (lo >> shift) << shift;
@@ -379,7 +443,9 @@ __global__ void __launch_bounds__(FIN_NT, 1) select_finish_kernel(const U* cand,
   }
   if (!out) return;
   const int64_t above = n - less - int64_t(eq);
-  if (held) {
+  if (above == 0) {
+    // the selected key is the largest of all: nothing to append
+  } else if (held) {
     uint32_t take = 0u;
 #pragma unroll
     for (int i = 0; i < V * E; i++) {
@@ -429,7 +495,7 @@ __global__ void __launch_bounds__(512) select_gather_kernel(const U* __restrict_
     st->cand_count = 0;
     st->gathered = 0;
     st->below = 0;
-    st->mode = SEL_MODE_CAND;
+    st->mode = SelMode<U>::CAND;
     st->ticket = 0;
     st->threshold = 0;
     st->threshold_hi = uint64_t(U(~U(0)));
@@ -688,7 +754,7 @@ __global__ void __launch_bounds__(256) partition_count_kernel(const U* keys, int
   const int lane = threadIdx.x & 31;
   const int64_t t = (int64_t(blockIdx.x) * 256 + threadIdx.x) >> 5;
   if (t >= ntiles) return;  // warp-uniform
-  const bool among = st->mode == SEL_MODE_CAND;
+  const bool among = st->mode == SelMode<U>::CAND;
   const WinTile w = tiles[t];
   const U* src = among ? cand + w.base : keys + t * T;
   const int m = among ? int(w.count) : int(n - t * T < T ? n - t * T : T);

@@ -3,6 +3,7 @@
 // keys, aux1: SelectState, aux2: tile counts), which the serving runtime binds to
 // slices of its arena.
 #pragma once
+#include <algorithm>
 #include <cmath>
 
 #include "sort_host.cuh"
@@ -97,9 +98,18 @@ inline int enqueue_window_select(hpcs_ctx* ctx, const U* d, int64_t n, int64_t r
   const int64_t width = (rhi >= S ? S : rhi + 1) - (rlo < 0 ? 0 : rlo);
   const int64_t expect = n < int64_t(4) * S || width >= S ? n : int64_t(double(width) / S * double(n));
   const bool finish = expect <= FIN_MAX_CANDIDATES;
+  // More candidates than the sample explains (its count of a window of `width` samples is off by one part
+  // in sqrt(width)): level 0 deals with them on all SMs.  But not a few that the cluster reads as fast: with
+  // both ends given their common digits need no level (select among 1 Mi f32 keys, half of them zero: 524 Ki
+  // candidates, 82 us in the cluster, 88 on all SMs), with the top open every level reads them (the 2^18
+  // largest of 1 Mi u32 keys, half of them the largest value: 112 and 92).
+  const int64_t few = open_top ? FIN_MAX_CANDIDATES * 3 / 4 : 2 * FIN_MAX_CANDIDATES;
+  const int64_t limit = std::max(few, int64_t(double(expect) * (1.0 + 6.0 / std::sqrt(double(width)))) + 32768);
   for (int shift = BITS - 8; shift >= 0; shift -= 8) {
-    if (!finish || shift == BITS - 8)
-      HPCS_CUDA(launch_chained(chained, select_level_kernel<U, KIND>, grid, SEL_NT, 0, s, d, n, c, rank, st, shift, open, finish ? 1 : 0));
+    if (!finish)
+      HPCS_CUDA(launch_chained(chained, select_level_kernel<U, KIND, false>, grid, SEL_NT, 0, s, d, n, c, rank, st, shift, open, limit));
+    else if (shift == BITS - 8)
+      HPCS_CUDA(launch_chained(chained, select_level_kernel<U, KIND, true>, grid, SEL_NT, 0, s, d, n, c, rank, st, shift, open, limit));
     if (shift == BITS - 8)
       HPCS_CUDA(launch_chained(chained, select_compact_kernel<U, KIND>, grid, SEL_NT, 0, s, d, n, cand, st, out, k));
   }
