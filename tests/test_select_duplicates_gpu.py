@@ -72,3 +72,33 @@ def test_misled_sample(ctx, dt, planted):
             got = a.copy()
             ctx.select_topk(got, k)
             np.testing.assert_array_equal(got, np.concatenate([a[a < v], a[a == v], a[a > v]]))
+
+
+def test_topk_time_with_copies():
+    """Half the keys equal to the largest: every copy is a candidate.  They are counted by all SMs, not by
+    one cluster (which took 16 times the uniform call here; by all SMs it is about 3 times)."""
+    import torch
+
+    c = native.Context(0)
+    s = native.torch_stream()
+    n, k = 1 << 26, 1000
+    uniform = torch.randint(0, 1 << 30, (n,), dtype=torch.int32, device="cuda")
+    copies = uniform.clone()
+    copies[::2] = (1 << 31) - 1
+    out = torch.empty(k, dtype=torch.int32, device="cuda")
+
+    def us(keys):
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            c.topk_largest_dev(keys, k, out, dtype="u32", stream=s)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b) * 1e3)
+        return sorted(times[2:])[2]
+
+    try:
+        assert us(copies) < 8 * us(uniform)
+    finally:
+        c.close()
