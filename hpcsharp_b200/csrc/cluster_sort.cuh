@@ -17,7 +17,10 @@
 // stores of ~32-key runs moved 5.6 bytes per clock and CTA (131072 u32 keys: 5800 of 13800 clocks a
 // pass).  An array of one slice never leaves its CTA: the reordered slice is the next pass's input,
 // and no cluster barrier is taken.
-// A pass whose keys all share one digit is left out.  The barriers are the cluster's hardware barrier
+// A pass whose keys all share one digit moves nothing.  The largest shape, whose sizes the look-back
+// passes sorted before with such passes left out, does not rank them either: its first pass finds the bits
+// that vary over all keys (the differences from the first key travel with the totals).  262,144 equal u32
+// keys: 56 us a call with four ranked passes, 19.5 so; smaller shapes would pay ~2 us of 30 for it.  The barriers are the cluster's hardware barrier
 // and every CTA takes the same ones, so no wait depends on data.
 #pragma once
 #include <cstdint>
@@ -48,7 +51,10 @@ struct ClusterSmem {
   static constexpr size_t OFF_TOT = OFF_MSK + MSK_BYTES;                              // [CTAS][256] totals
   static constexpr size_t OFF_GBASE = OFF_TOT + size_t(CS_MAX_CTAS) * RADIX * 4;      // global base - local
   static constexpr size_t OFF_WSUM = OFF_GBASE + RADIX * 4;
-  static constexpr size_t BYTES = OFF_WSUM + 32 * 4;
+  static constexpr bool LOOK = KPT >= 32;  // leaves passes on constant digits out
+  static constexpr size_t OFF_WBITS = OFF_WSUM + 32 * 4;                        // [NW] varying bits of a warp's keys
+  static constexpr size_t OFF_CBITS = OFF_WBITS + size_t(NW) * sizeof(U);       // [CTAS] of a CTA's
+  static constexpr size_t BYTES = LOOK ? OFF_CBITS + size_t(CS_MAX_CTAS) * sizeof(U) : OFF_WBITS;
   static_assert(SLICE < 65536, "offsets are kept in 16 bits");
 };
 
@@ -68,6 +74,14 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t a, uint32_t rank) {
 }
 __device__ __forceinline__ void cluster_store(uint32_t a, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_store(uint32_t a, uint64_t v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+// OR over a warp's values.
+__device__ __forceinline__ uint32_t warp_or(uint32_t v) { return __reduce_or_sync(0xFFFFFFFFu, v); }
+__device__ __forceinline__ uint64_t warp_or(uint64_t v) {
+  return uint64_t(warp_or(uint32_t(v >> 32))) << 32 | warp_or(uint32_t(v));
 }
 // Keys that other CTAs wrote: through L2, never from a stale L1 line.
 __device__ __forceinline__ uint32_t ld_cg(const uint32_t* p) { return __ldcg(p); }
@@ -89,6 +103,8 @@ __global__ void __launch_bounds__(CS_NT, 1) cluster_sort_kernel(U* keys, uint32_
   uint32_t* s_tot = reinterpret_cast<uint32_t*>(smem + L::OFF_TOT);
   uint32_t* s_gbase = reinterpret_cast<uint32_t*>(smem + L::OFF_GBASE);
   uint32_t* s_wsum = reinterpret_cast<uint32_t*>(smem + L::OFF_WSUM);
+  U* s_wbits = reinterpret_cast<U*>(smem + L::OFF_WBITS);
+  U* s_cbits = reinterpret_cast<U*>(smem + L::OFF_CBITS);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t* cnt_w = s_cnt + warp * RS;
   const uint16_t* off_w = s_off + warp * L::OS;
@@ -107,9 +123,12 @@ __global__ void __launch_bounds__(CS_NT, 1) cluster_sort_kernel(U* keys, uint32_
   U* buf = reinterpret_cast<U*>(smem + L::OFF_BUF);
   uint32_t* vbuf = reinterpret_cast<uint32_t*>(smem + L::OFF_BUF + L::KEYS_BYTES);
   for (int i = lane; i < RADIX; i += 32) cnt_w[i] = 0u;
+  const bool look = L::LOOK && skip_trivial;
+  U varies = U(~U(0));  // the bits that differ among the keys (every bit until the first pass has looked)
   for (int p = 0; p < P; p++) {
+    if (L::LOOK && (uint32_t(varies >> (8 * p)) & 0xFFu) == 0u) continue;  // uniform over the cluster
     const Digit<U, KIND> dig(8 * p);
-    const bool last = p == P - 1;
+    bool last = p == P - 1;
     __syncwarp();
 
     // ---- load (warp-striped) and rank within the warp --------------------------------
@@ -130,6 +149,15 @@ __global__ void __launch_bounds__(CS_NT, 1) cluster_sort_kernel(U* keys, uint32_
         key[i] = idx < cnt ? ld_cg(keys + lo + idx) : U(0);
         if (PAIRS) val[PAIRS ? i : 0] = idx < cnt ? ld_cg(vals + lo + idx) : 0u;
       }
+    }
+    if (look && p == 0) {
+      const U first = ld_cg(keys);
+      U diff = U(0);
+#pragma unroll
+      for (int i = 0; i < KPT; i++)
+        if (wbase + i * 32 + lane < cnt) diff |= key[i] ^ first;
+      diff = warp_or(diff);
+      if (lane == 0) s_wbits[warp] = diff;
     }
 #pragma unroll
     for (int i = 0; i < (KPT + 1) / 2; i++) rank[i] = 0u;
@@ -163,6 +191,11 @@ __global__ void __launch_bounds__(CS_NT, 1) cluster_sort_kernel(U* keys, uint32_
         const uint32_t slot = smem_u32(s_tot + cta * RADIX + sd);
         for (uint32_t r = uint32_t(sq); r < ctas; r += uint32_t(G)) cluster_store(cluster_addr(slot, r), total);
         __syncwarp();
+        if (look && p == 0 && warp == L::NW - 1) {
+          const U diff = warp_or(lane < L::NW ? s_wbits[lane] : U(0));
+          if (lane < int(ctas)) cluster_store(cluster_addr(smem_u32(s_cbits + cta), uint32_t(lane)), diff);
+          __syncwarp();
+        }
       }
       uint32_t di = total;  // inclusive over this warp's digits (lanes G apart)
 #pragma unroll
@@ -214,6 +247,14 @@ __global__ void __launch_bounds__(CS_NT, 1) cluster_sort_kernel(U* keys, uint32_
     }
     cluster_arrive();  // (the totals have long arrived: the release does not wait for them)
     cluster_wait();    // every CTA's totals are here, and every CTA's keys are in registers
+    if (look) {
+      if (p == 0) {
+        varies = warp_or(lane < int(ctas) ? s_cbits[lane] : U(0));
+        // floats of both signs: the order flips every bit of the negative ones
+        if (KIND == KIND_FLOAT && (varies >> (8 * P - 1)) != 0) varies = U(~U(0));
+      }
+      last = last || U(varies >> (8 * (p < P - 1 ? p + 1 : 0))) == 0;
+    }
 
     // ---- global bases: digit starts over all slices + the slices before this one -------
     uint32_t all = 0, pre = 0;
