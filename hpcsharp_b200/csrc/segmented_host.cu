@@ -92,8 +92,7 @@ int seg_build_groups(const hpcs_seg_tuning& tuning, int few_tiled, const hpcs_se
     group_bytes[WIDE] += group_bytes[NARROW];
     group_bytes[NARROW] = 0.0;
   }
-  // groups in decreasing total bytes (the heaviest is launched first, on the caller's
-  // stream), arrays within a group largest first
+  // groups in decreasing total bytes, arrays within a group largest first
   std::vector<int> vorder(NG);
   std::iota(vorder.begin(), vorder.end(), 0);
   std::stable_sort(vorder.begin(), vorder.end(), [&](int a, int b) { return group_bytes[a] > group_bytes[b]; });
@@ -128,7 +127,37 @@ int seg_build_groups(const hpcs_seg_tuning& tuning, int few_tiled, const hpcs_se
       scratch += (size_t(sg.n) * w + 255) / 256 * 256;
     }
   }
+  if (!groups.empty()) seg_deal(table.data(), groups, hpcs_ctx::SEG_BRANCHES);
   return HPCS_OK;
+}
+
+void seg_deal(const SegDesc* table, std::vector<SegGroup>& groups, int branches) {
+  const int ng = int(groups.size());
+  std::vector<double> longest(groups.size(), 0.0), share(groups.size(), 0.0), bytes(groups.size(), 0.0);
+  for (int g = 0; g < ng; g++) {
+    for (int j = groups[g].first; j < groups[g].first + groups[g].count; j++) {
+      const int passes = key_bytes(table[j].dtype);
+      const double kib = double(table[j].n) * passes / 1024.0;
+      longest[g] = std::max(longest[g], passes * (1.5 + 0.12 * kib));
+      share[g] += 0.0009 * passes * kib;
+      bytes[g] += kib;
+    }
+  }
+  const bool balance = std::accumulate(share.begin(), share.end(), 0.0) < 1.75 * *std::max_element(longest.begin(), longest.end());
+  std::vector<int> order(groups.size());
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return balance ? longest[a] + share[a] > longest[b] + share[b] : bytes[a] > bytes[b];
+  });
+  std::vector<double> load(size_t(branches) + 1, 0.0);
+  std::vector<SegGroup> dealt;
+  for (int i = 0; i < ng; i++) {
+    const int g = order[i];
+    groups[g].stream = balance ? int(std::min_element(load.begin(), load.end()) - load.begin()) : i == 0 ? 0 : 1 + (i - 1) % std::min(branches, 3);
+    load[groups[g].stream] += longest[g] + share[g];
+    dealt.push_back(groups[g]);
+  }
+  groups = std::move(dealt);
 }
 
 void seg_relocate(std::vector<SegDesc>& table, const std::vector<SegGroup>&, void* base) {
@@ -142,19 +171,20 @@ int launch_groups_mode(hpcs_ctx* ctx, const SegDesc* d_desc, const std::vector<S
                        uint32_t* d_queues, cudaStream_t s) {
   int rc;
   const int ng = int(groups.size());
-  if (ng > 1) {
+  int helpers = 0;  // the first ones are in use (seg_deal)
+  for (const SegGroup& g : groups) helpers = std::max(helpers, g.stream);
+  if (helpers > 0) {
     if ((rc = ensure_seg_streams(ctx)) != HPCS_OK) return rc;
     HPCS_CUDA(cudaEventRecord(ctx->seg_fork, s));
-    for (int b = 0; b < hpcs_ctx::SEG_BRANCHES && b < ng - 1; b++)
-      HPCS_CUDA(cudaStreamWaitEvent(ctx->seg_streams[b], ctx->seg_fork, 0));
+    for (int b = 0; b < helpers; b++) HPCS_CUDA(cudaStreamWaitEvent(ctx->seg_streams[b], ctx->seg_fork, 0));
   }
   for (int g = 0; g < ng; g++) {
-    cudaStream_t st = g == 0 ? s : ctx->seg_streams[(g - 1) % hpcs_ctx::SEG_BRANCHES];
+    cudaStream_t st = groups[g].stream == 0 ? s : ctx->seg_streams[groups[g].stream - 1];
     if ((rc = launch_seg_variant<MODE>(ctx, groups[g].variant, groups[g].large, d_desc + groups[g].first,
                                        groups[g].count, d_queues + g, st, groups[g].longest)) != HPCS_OK)
       return rc;
   }
-  for (int b = 0; b < hpcs_ctx::SEG_BRANCHES && b < ng - 1; b++) {
+  for (int b = 0; b < helpers; b++) {
     HPCS_CUDA(cudaEventRecord(ctx->seg_join[b], ctx->seg_streams[b]));
     HPCS_CUDA(cudaStreamWaitEvent(s, ctx->seg_join[b], 0));
   }

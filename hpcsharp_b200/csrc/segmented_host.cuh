@@ -139,7 +139,19 @@ struct SegGroup {
   int first;
   int count;
   int64_t longest;  // bytes of its longest array where one array's own time counts, else 0
+  int stream = 0;   // 0: the caller's, else a helper
 };
+// Orders the groups for launching and gives each its stream.  Launches on one stream run one after the
+// other.  Expected times: the longest array's passes in one CTA (0.12 us per KiB; tiles of 64 KiB take
+// 6-9.4 us) and the group's share of the full GPU (0.9 ns per KiB and pass).
+//   one array's time counts (all groups' shares add up to less than 1.75 of it): the longest first, each on
+//     the stream with the least to do, so that nothing waits behind the longest;
+//   else in decreasing bytes, dealt out in turn.
+// Whole batches, us, in turn / balanced, by shares over longest time: 0.1 133 / 111, 0.5 142 / 116, 1.0 164 /
+// 112, 1.3 166 / 136, 1.4 419 / 417, 1.95 439 / 449, 2.1 124 / 134, 2.4 765 / 788.  Balanced over three helpers
+// 68 short arrays take 40 us, over four 33, over seven 32 (but 161 in place of 136 at 1.3); in turn the three
+// that the batched sort always had.
+void seg_deal(const SegDesc* table, std::vector<SegGroup>& groups, int branches);
 
 // Whether variant v sorts an array of n keys of width w with its tiled (scratch) path.
 inline bool seg_variant_large(int v, int64_t n, int key_bytes) {

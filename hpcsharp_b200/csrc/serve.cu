@@ -334,6 +334,7 @@ void launch_batch(hpcs_server* sv) {
     g.variant = SEG_WIDE_TILES;
     g.longest = longest.n * dtype_bytes(longest.dtype);
   }
+  if (!groups.empty()) seg_deal(sv->host_table, groups, hpcs_ctx::SEG_BRANCHES);
   cudaMemcpyAsync(d_table, sv->host_table, n * sizeof(SegDesc), cudaMemcpyHostToDevice, s);
   c->last_stream = s;
   int rc = seg_launch_groups(c, d_table, groups, d_queues, s);

@@ -72,7 +72,7 @@ struct hpcs_ctx {
   // and events that run the launches of different variants concurrently
   hpcs_seg_tuning seg_tuning{};
   bool seg_tuning_set = false;  // by the caller: followed as it is
-  static constexpr int SEG_BRANCHES = 3;
+  static constexpr int SEG_BRANCHES = 4;
   cudaStream_t seg_streams[SEG_BRANCHES] = {};
   cudaEvent_t seg_fork = nullptr;
   cudaEvent_t seg_join[SEG_BRANCHES] = {};

@@ -1,0 +1,82 @@
+"""How a batch's launches are spread over the streams: a batch bound by one array's time (a few long arrays
+among many short ones of every class), one bound by the GPU's throughput, batches of one and of two
+launches; as a planned call and as a direct one.  Bits against the oracle, and the time of the first kind:
+nothing may run behind its longest array."""
+import numpy as np
+import pytest
+
+from hpcsharp_b200 import datagen, native
+
+pytestmark = pytest.mark.gpu
+
+SETS = {
+    "one array's time": [(100, 40), (200, 40), (400, 30), (1500, 30), (3500, 20), (7000, 20), (13_000, 6)],
+    "throughput": [(100, 400), (400, 300), (1500, 300), (3500, 300), (7000, 300), (13_000, 330)],
+    "one launch": [(100, 5)],
+    "two launches": [(100, 5), (20_000, 2)],
+}
+
+
+def _make(lengths, dtypes):
+    import torch
+
+    arrays, segs, keep = [], [], []
+    i = 0
+    for n, count in lengths:
+        for _ in range(count):
+            dt = dtypes[i % len(dtypes)]
+            a = datagen.by_name(dt, n + i % 7, seed=i)
+            t = torch.from_numpy(a.view(np.uint8)).cuda()
+            arrays.append((a, t))
+            segs.append(((t.data_ptr(), a.size), dt))
+            i += 1
+    return arrays, segs
+
+
+@pytest.mark.parametrize("kind", sorted(SETS))
+@pytest.mark.parametrize("planned", [True, False], ids=["plan", "direct"])
+def test_batch_streams(ctx, orc, kind, planned):
+    import torch
+
+    arrays, segs = _make(SETS[kind], ["u32", "f32", "u64", "i64"])
+    torch.cuda.synchronize()
+    if planned:
+        plan = ctx.segplan(segs)
+        plan.execute()
+        ctx.synchronize()
+        plan.close()
+    else:
+        ctx.sort_segmented_dev(segs)
+        ctx.synchronize()
+    for a, t in arrays:
+        want = a.copy()
+        orc.sort_radix_lsd(want)
+        assert np.array_equal(t.cpu().numpy(), want.view(np.uint8)), (kind, a.dtype, a.size)
+
+
+def test_nothing_behind_the_longest(ctx):
+    """Six 13,000-key u64 arrays among 180 shorter ones of every class take little longer than alone (1.1
+    times; with two groups behind them 1.4 times)."""
+    import torch
+
+    def us(segs):
+        plan = ctx.segplan(segs)
+        s = native.torch_stream()
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(10):
+                plan.execute(stream=s)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b) * 100)
+        plan.close()
+        return sorted(times)[2]
+
+    lengths = SETS["one array's time"]
+    keep, segs = _make(lengths, ["u32", "f32", "u64", "u64"])
+    long_, alone = _make([(13_000, 6)], ["u64"])
+    rest = [s for s in segs if s[0][1] < 13_000]
+    assert us(rest + alone) < 1.25 * us(alone)
+    del keep, long_
