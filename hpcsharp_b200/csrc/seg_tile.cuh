@@ -250,24 +250,26 @@ __device__ __forceinline__ void seg_tile_sort(U* keys, U* scratch, int64_t n, in
     if (tid < RADIX) s_run[tid] = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? s_wsum[lane] : 0u) + incl - c;
     const RunDigit<U> dig(kind, 8 * p);
     const bool staged = aligned || src == scratch;  // (scratch is aligned)
-    if (staged && tid == 0) stage_tile<U, false, TILE>(smem + L::OFF_STAGE, 0, s_mbar, src, nullptr, n, 0);
+    // a pass's first tile is loaded directly, the second staged meanwhile
+    if (staged && ntiles > 1 && tid == 0) stage_tile<U, false, TILE>(smem + L::OFF_STAGE, 0, s_mbar, src, nullptr, n, 1);
     __syncthreads();  // running starts ready; s_wsum may be rewritten
     for (int t = 0; t < ntiles; t++) {
       const int64_t tb = int64_t(t) * TILE;
       const int tile_n = int(n - tb < TILE ? n - tb : TILE);
       U key[KPT];
-      if (staged) {
+      const bool bulked = staged && t > 0;
+      if (bulked) {
         if (!mbar_wait_bounded(s_mbar, phase, spin_limit_ns) && lane == 0) atomicOr(err, uint32_t(DERR_TMA_TIMEOUT));
         phase ^= 1u;
       }
-      const int bulk = staged ? int((int64_t(tile_n) * int64_t(sizeof(U))) & ~int64_t(15)) / int(sizeof(U)) : 0;
+      const int bulk = bulked ? int((int64_t(tile_n) * int64_t(sizeof(U))) & ~int64_t(15)) / int(sizeof(U)) : 0;
 #pragma unroll
       for (int i = 0; i < KPT; i++) {
         const int idx = wbase + i * 32 + lane;
         key[i] = idx < bulk ? stage[idx] : (idx < tile_n ? src[tb + idx] : U(0));
       }
       fence_proxy_async_smem();  // the stage buffer was read; the next bulk copy overwrites it
-      seg_tile_reorder<U, NT, KPT4, MODE>(key, tile_n, dig, smem, src, n, staged && t + 1 < ntiles ? t + 1 : -1);
+      seg_tile_reorder<U, NT, KPT4, MODE>(key, tile_n, dig, smem, src, n, bulked && t + 1 < ntiles ? t + 1 : -1);
       // ---- coalesced per-digit runs; every destination is checked against n ------------------
 #pragma unroll
       for (int b = 0; b < KPT; b += BATCH) {
