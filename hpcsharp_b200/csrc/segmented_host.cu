@@ -82,11 +82,12 @@ int seg_build_groups(const hpcs_seg_tuning& tuning, int few_tiled, const hpcs_se
     group_bytes[var[i]] += double(segs[i].n) * w;
   }
   // Few tiled arrays: one array's own time is what counts, and the wide shape sorts an array in about
-  // half the narrow one's.  The line: the narrow shape would hold them all at once (two CTAs per SM), so
-  // its better throughput does not come to bear (whole batches, us, narrow / wide, by tiled arrays: 7
-  // 153 / 112, 74 266 / 220, 179 359 / 232, 263 416 / 306, 292 343 / 327, 430 402 / 454, 597 523 / 609).
+  // half the narrow one's.
   constexpr int NARROW = 2 * SEG_NARROW_TILES + 1, WIDE = 2 * SEG_WIDE_TILES + 1;
-  const bool few = std::count(var.begin(), var.end(), NARROW) + std::count(var.begin(), var.end(), WIDE) <= few_tiled;
+  std::vector<int64_t> tiled;
+  for (int64_t i = 0; i < nsegs; i++)
+    if (var[i] == NARROW || var[i] == WIDE) tiled.push_back(segs[i].n * key_bytes(segs[i].dtype));
+  const bool few = int64_t(tiled.size()) <= few_tiled && seg_wide_pays(tiled, few_tiled / 2);
   if (few) {
     std::replace(var.begin(), var.end(), NARROW, WIDE);
     group_bytes[WIDE] += group_bytes[NARROW];

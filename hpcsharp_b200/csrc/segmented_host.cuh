@@ -158,13 +158,29 @@ inline bool seg_variant_large(int v, int64_t n, int key_bytes) {
   return SEG_VARIANTS[v].kind == 1 && n > seg_variant_tile_keys(v, key_bytes);
 }
 
-// Orders the descriptors by (variant, bytes descending), fills `groups`, and returns through
-// `scratch` the bytes of scratch the block-level arrays longer than one tile need (their
-// scratch fields hold offsets until seg_relocate).
 // The arrays of the narrow tiled shape up to which a batch runs them in the wide one: what the narrow
 // shape holds at once.  A table set by the caller is followed as it is (-1).
 inline int seg_few_tiled(const hpcs_ctx* ctx) { return ctx->seg_tuning_set ? -1 : 2 * ctx->sms; }
-// Up to `few_tiled` arrays of the narrow tiled shape run in the wide one (negative: the table as it is).
+// Whether up to two tiled arrays per SM, of these sizes in bytes, are sorted sooner in the wide shape (one
+// per SM) than in the narrow one (two).  An array's time goes with its bytes (key width x digits); beside
+// another on its SM a narrow one takes 1.85 times a wide one's.  Wide: the longest, an SM's share of all, or
+// the two that share an SM where there are more arrays than SMs.  (us, narrow / wide, 148 SMs: whole batches
+// of mixed lengths with 179 tiled arrays 359 / 232, 263 416 / 306, 292 343 / 327; equal u32 arrays of 20,000
+// keys: 148 82 / 66, 160 104 / 113, 296 110 / 120; u64 of 13,000: 124 / 101, 167 / 182, 176 / 193.)
+inline bool seg_wide_pays(std::vector<int64_t> bytes, int sms) {
+  if (bytes.empty()) return true;
+  std::sort(bytes.begin(), bytes.end(), [](int64_t a, int64_t b) { return a > b; });
+  double total = 0.0;
+  for (int64_t b : bytes) total += double(b);
+  double wide = std::max(double(bytes[0]), total / sms);
+  if (int64_t(bytes.size()) > sms) wide = std::max(wide, double(bytes[size_t(sms) - 1]) + double(bytes[size_t(sms)]));
+  return wide <= 1.85 * std::max(double(bytes[0]), total / (2.0 * sms));
+}
+// Orders the descriptors by (variant, bytes descending), fills `groups`, and returns through
+// `scratch` the bytes of scratch the block-level arrays longer than one tile need (their
+// scratch fields hold offsets until seg_relocate).
+// Up to `few_tiled` arrays of the narrow tiled shape run in the wide one where that pays (negative: the table
+// as it is).
 int seg_build_groups(const hpcs_seg_tuning& tuning, int few_tiled, const hpcs_segment* segs, int64_t nsegs,
                      std::vector<SegDesc>& table, std::vector<SegGroup>& groups, size_t& scratch);
 void seg_relocate(std::vector<SegDesc>& table, const std::vector<SegGroup>& groups, void* base);

@@ -330,6 +330,9 @@ void launch_batch(hpcs_server* sv) {
   // few tiled arrays take the wide tiled shape, as in a batched sort
   for (SegGroup& g : groups) {
     if (g.variant != SEG_NARROW_TILES || !g.large || g.count > seg_few_tiled(c)) continue;
+    std::vector<int64_t> bytes;
+    for (int j = g.first; j < g.first + g.count; j++) bytes.push_back(sv->host_table[j].n * dtype_bytes(sv->host_table[j].dtype));
+    if (!seg_wide_pays(bytes, c->sms)) continue;
     const SegDesc& longest = sv->host_table[g.first];
     g.variant = SEG_WIDE_TILES;
     g.longest = longest.n * dtype_bytes(longest.dtype);
