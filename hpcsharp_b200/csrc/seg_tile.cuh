@@ -46,8 +46,8 @@ struct SegTileSmem {
   static_assert(NT * KPT4 < 65536, "offsets are kept in 16 bits");
 };
 
-// Digit of one pass for a key order known at run time (the three orders of one key width share their
-// code: an SM runs arrays of several types at once, and six copies of the unrolled loops missed the
+// Digit of one pass for a key order known at run time (but for u64 in the wide shape the three orders of one
+// key width share their code: an SM runs arrays of several types at once, and six copies of the unrolled loops missed the
 // instruction cache, 2 of ~10 stall cycles per instruction).  x ^ top ^ (sign & flip): unsigned keys
 // change nothing, signed keys the sign bit, floats the sign bit or, when negative, every bit.
 template <class U>
@@ -329,7 +329,13 @@ __global__ void __launch_bounds__(NT, 512 / NT) seg_tile_kernel(SegParams prm) {
     const SegDesc sd = prm.segs[sidx];
     if (sd.n <= 1) continue;
     const int kind = sd.dtype % 3;  // u32, i32, f32, u64, i64, f64: unsigned, signed, float
-    if (sd.dtype >= 3)
+    // The wide shape, one array at a time on its SM, has a copy for unsigned 8-byte keys without the order
+    // transform, which every digit of theirs paid: one array of 13,000 keys 94 -> 86 us, 148 of 50,000 323 ->
+    // 300 (u32 arrays, whose code shares the registers, 0-3% slower).  Two arrays per SM share their code.
+    if (NT == 512 && sd.dtype == 3)
+      seg_tile_sort<uint64_t, NT, KPT4, MODE>(static_cast<uint64_t*>(sd.keys), static_cast<uint64_t*>(sd.scratch), sd.n, KIND_UNSIGNED, smem,
+                                    prm.err, prm.spin_limit_ns, phase);
+    else if (sd.dtype >= 3)
       seg_tile_sort<uint64_t, NT, KPT4, MODE>(static_cast<uint64_t*>(sd.keys), static_cast<uint64_t*>(sd.scratch), sd.n, kind, smem,
                                     prm.err, prm.spin_limit_ns, phase);
     else
