@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <mutex>
@@ -287,10 +288,10 @@ int launch_lookback_tiles(hpcs_ctx* ctx, SortArgs args, bool chained, cudaStream
 }
 
 template <class U, int KIND, class V, int MODE>
-int launch_lookback_passes(hpcs_ctx* ctx, const SortArgs& args, bool chained, cudaStream_t s) {
+int launch_lookback_passes(hpcs_ctx* ctx, const SortArgs& args, int kpt, bool chained, cudaStream_t s) {
   constexpr int LARGE = SortConfig<U, V, MODE>::KPT;
   constexpr bool ONE = MODE == RANK_PEER_MASK;
-  switch (lookback_kpt<U, V, MODE>(args.n, ctx->sms)) {
+  switch (kpt) {
     case 8: return launch_lookback_tiles<U, KIND, V, MODE, ONE ? LARGE : 8>(ctx, args, chained, s);
     case 16: return launch_lookback_tiles<U, KIND, V, MODE, ONE ? LARGE : 16>(ctx, args, chained, s);
     default: return launch_lookback_tiles<U, KIND, V, MODE, LARGE>(ctx, args, chained, s);
@@ -396,6 +397,19 @@ int enqueue_cluster_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cuda
   return HPCS_OK;
 }
 
+// Whether the sort's rows (and its plan) fit the context's budget, or the slices it was lent.
+inline bool rows_fit(const hpcs_ctx* ctx, size_t row_bytes0, size_t row_bytes1) {
+  const DevBuf* bufs[3] = {&ctx->status0, &ctx->status1, &ctx->plan};
+  const size_t want[3] = {row_bytes0, row_bytes1, sizeof(SortPlan)};
+  size_t held = ctx->held_bytes;
+  for (int i = 0; i < 3; i++) {
+    if (bufs[i]->bytes >= want[i]) continue;
+    if (bufs[i]->borrowed) return false;
+    held += std::max(want[i], size_t(256)) - bufs[i]->bytes;
+  }
+  return ctx->cfg.pool_bytes <= 0 || held <= size_t(ctx->cfg.pool_bytes);
+}
+
 // Enqueue a full LSD sort of n keys (and optional 4-byte items) in device memory.
 // keys/vals are sorted in place (with scratch B owned by the context).
 template <class U, int KIND, class V>
@@ -412,8 +426,6 @@ int enqueue_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t
   const bool capturing = cap != cudaStreamCaptureStatusNone;
   const bool ordered = ctx->rank_mode == RANK_ORDERED_ATOMIC;
   int rc;
-  if ((rc = ensure(ctx, ctx->keys_b, size_t(n) * sizeof(U))) != HPCS_OK) return rc;
-  if (PAIRS && (rc = ensure(ctx, ctx->vals_b, size_t(n) * 4)) != HPCS_OK) return rc;
   // small sorts: one cluster launch (not when a pass scheme is forced)
   if (ctx->cfg.pass_scheme == HPCS_PASSES_AUTO) {
     bool done = false;
@@ -421,20 +433,8 @@ int enqueue_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t
                  : enqueue_cluster_sort<U, KIND, V, RANK_PEER_MASK>(ctx, keys, vals, n, s, &done);
     if (rc != HPCS_OK || done) return rc;
   }
-  const bool lookback = ctx->cfg.pass_scheme != HPCS_PASSES_CHUNKED;
-  // the look-back launches are chained: each pass's CTAs start as the last pass's finish (u32 sorts,
-  // us, plain / chained launches: 150 Ki keys 69 / 51, 1 Mi 75 / 61, 10 M 181 / 167)
-  const bool chained = lookback && !capturing;
-  const int64_t unit = ordered ? int64_t(CA::NT) * lookback_kpt<U, V, RANK_ORDERED_ATOMIC>(n, ctx->sms)
-                               : int64_t(CP::NT) * lookback_kpt<U, V, RANK_PEER_MASK>(n, ctx->sms);
-  const int64_t num_tiles = lookback ? (n + unit - 1) / unit : 0;
-  ChunkGeometry geo{0, 0, 0};
-  if (!lookback) {
-    using SA = ChunkShape<U, V, RANK_ORDERED_ATOMIC>;
-    using SP = ChunkShape<U, V, RANK_PEER_MASK>;
-    const int cap = ordered ? SA::MAX_RANGES : SP::MAX_RANGES;
-    geo = chunk_geometry(n, ordered ? SA::TILE : SP::TILE, ctx->sms < cap ? ctx->sms : cap);
-  }
+  if ((rc = ensure(ctx, ctx->keys_b, size_t(n) * sizeof(U))) != HPCS_OK) return rc;
+  if (PAIRS && (rc = ensure(ctx, ctx->vals_b, size_t(n) * 4)) != HPCS_OK) return rc;
 
   // 16-byte alignment is required by the bulk copies; unaligned callers go through A'.
   U* a = keys;
@@ -452,10 +452,41 @@ int enqueue_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t
     HPCS_CUDA(cudaMemcpyAsync(va, vals, size_t(n) * 4, cudaMemcpyDeviceToDevice, s));
   }
   constexpr int P = int(sizeof(U));
-  const size_t status_bytes = lookback ? size_t(num_tiles) * RADIX * 4 : size_t(geo.chunks) * (P + 3) * RADIX * 4;
-  if ((rc = ensure(ctx, ctx->status0, status_bytes)) != HPCS_OK) return rc;
-  if (lookback && (rc = ensure(ctx, ctx->status1, status_bytes)) != HPCS_OK) return rc;
-  if ((rc = ensure(ctx, ctx->plan, sizeof(SortPlan))) != HPCS_OK) return rc;
+  // The passes: look-back with the tile for n, look-back with the large tile, chunked (unless a scheme is
+  // forced); the first whose rows fit.  The later ones are slower and take less scratch: 2^28 u32 keys 26 MiB
+  // of look-back rows, 1 MiB of count tables; 1 Mi keys 128 Ki + 128 Ki of rows, with the large tile 52 + 52.
+  const int tile_kpt[2] = {ordered ? lookback_kpt<U, V, RANK_ORDERED_ATOMIC>(n, ctx->sms) : CP::KPT, ordered ? CA::KPT : CP::KPT};
+  ChunkGeometry geo{0, 0, 0};
+  int64_t num_tiles = 0;
+  int kpt = 0;  // 0: chunked passes
+  const int first = ctx->cfg.pass_scheme == HPCS_PASSES_CHUNKED ? 2 : 0, last = ctx->cfg.pass_scheme == HPCS_PASSES_LOOKBACK ? 1 : 2;
+  for (int option = first; option <= last; option++) {
+    kpt = option < 2 ? tile_kpt[option] : 0;
+    size_t rows[2];
+    if (kpt) {
+      const int64_t unit = int64_t(ordered ? CA::NT : CP::NT) * kpt;
+      num_tiles = (n + unit - 1) / unit;
+      rows[0] = rows[1] = size_t(num_tiles) * RADIX * 4;
+    } else {
+      using SA = ChunkShape<U, V, RANK_ORDERED_ATOMIC>;
+      using SP = ChunkShape<U, V, RANK_PEER_MASK>;
+      const int cap = ordered ? SA::MAX_RANGES : SP::MAX_RANGES;
+      geo = chunk_geometry(n, ordered ? SA::TILE : SP::TILE, ctx->sms < cap ? ctx->sms : cap);
+      num_tiles = 0;
+      rows[0] = size_t(geo.chunks) * (P + 3) * RADIX * 4;
+      rows[1] = 0;
+    }
+    if (option < last && !rows_fit(ctx, rows[0], rows[1])) continue;
+    rc = ensure(ctx, ctx->status0, rows[0]);
+    if (rc == HPCS_OK && rows[1]) rc = ensure(ctx, ctx->status1, rows[1]);
+    if (rc == HPCS_OK) rc = ensure(ctx, ctx->plan, sizeof(SortPlan));
+    if (rc != HPCS_ERR_OOM) break;  // (the device itself may be full)
+  }
+  if (rc != HPCS_OK) return rc;
+  const bool lookback = kpt != 0;
+  // the look-back launches are chained: each pass's CTAs start as the last pass's finish (u32 sorts,
+  // us, plain / chained launches: 150 Ki keys 69 / 51, 1 Mi 75 / 61, 10 M 181 / 167)
+  const bool chained = lookback && !capturing;
 
   SortArgs args{};
   args.keys_a = a;
@@ -493,8 +524,8 @@ int enqueue_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t
     rc = ordered ? launch_chunk_passes<U, KIND, V, RANK_ORDERED_ATOMIC>(ctx, args, s)
                  : launch_chunk_passes<U, KIND, V, RANK_PEER_MASK>(ctx, args, s);
   else
-    rc = ordered ? launch_lookback_passes<U, KIND, V, RANK_ORDERED_ATOMIC>(ctx, args, chained, s)
-                 : launch_lookback_passes<U, KIND, V, RANK_PEER_MASK>(ctx, args, chained, s);
+    rc = ordered ? launch_lookback_passes<U, KIND, V, RANK_ORDERED_ATOMIC>(ctx, args, kpt, chained, s)
+                 : launch_lookback_passes<U, KIND, V, RANK_PEER_MASK>(ctx, args, kpt, chained, s);
   if (rc != HPCS_OK) return rc;
   // finalize: result back into the caller's buffer if it ended in B; collect errors
   {
