@@ -172,65 +172,92 @@ __global__ void probe_check_kernel(const uint32_t* keys, const uint32_t* items, 
   if (v) atomicAdd(bad, v);
 }
 
-// Runs the shipping ordered-atomic pass kernels -- the chunked passes and the look-back passes,
-// keys only and with items -- on inputs with many equal digits per warp instruction and checks
-// the results for order and stability.  Any violation sends the context to the peer-mask
-// ranking, which is defined by PTX.  The same code generation and occupancy as a real sort: the
-// probe calls the sort's own enqueue functions.
-int probe_shipping_kernels(hpcs_ctx* ctx, int* ok) {
-  // the look-back passes take their middle, large and small tile at these sizes
-  constexpr int64_t sizes[3] = {(int64_t(1) << 20) + 12345, (int64_t(5) << 19) + 12345, 300007};
+// The sorts that the probe runs: every kernel shape of 4-byte unsigned keys (tests/test_probe_cpu.py holds
+// the list against the shapes that the sorts take).
+struct ProbeSort {
+  int scheme;
+  int64_t n;
+};
+std::vector<ProbeSort> probe_sorts(int sms, bool items) {
+  constexpr int64_t NT = SortConfig<uint32_t, NoValue, RANK_ORDERED_ATOMIC>::NT;
+  std::vector<ProbeSort> v = {{HPCS_PASSES_CHUNKED, (int64_t(1) << 20) + 12345},
+                              // the look-back passes' small, middle and large tile
+                              {HPCS_PASSES_LOOKBACK, sms * NT * 4 + 7},
+                              {HPCS_PASSES_LOOKBACK, sms * NT * 8 + 12345},
+                              {HPCS_PASSES_LOOKBACK, sms * NT * 32 + 12345},
+                              // the one-launch sort in one CTA (4, 8 and 16 keys per thread) and in clusters (8, 16, 32)
+                              {HPCS_PASSES_AUTO, 1500},
+                              {HPCS_PASSES_AUTO, 3501},
+                              {HPCS_PASSES_AUTO, 7003},
+                              {HPCS_PASSES_AUTO, 50003},
+                              {HPCS_PASSES_AUTO, 100003}};
+  if (!items) v.push_back({HPCS_PASSES_AUTO, 200003});
+  return v;
+}
+// Lengths of the tiled arrays of the batched sort that the probe runs: the wide shape's two tiles and, with
+// `narrow`, the narrow shape.
+struct ProbeSegment {
+  int64_t n;
+  bool narrow;
+};
+constexpr ProbeSegment PROBE_SEGMENTS[] = {{23003, false}, {30011, false}, {30011, true}};
+
+// Runs the shipping ordered-atomic kernels -- the chunked and the look-back passes, the one-launch small
+// sort, each with and without items, and the batched sort's tiled kernel -- on inputs with many equal digits
+// per warp instruction and checks the results for order and stability (an unstable pass of a sort
+// without items shows in the order).  Of the digit values' numbers, 20 and 4 go through the atomics (4
+// leave 8 lanes of a warp on one counter), 3 through the votes of a frequent value.  Any violation sends
+// the context to the peer-mask ranking, which is defined by PTX.  The same code generation and occupancy as a
+// real sort: the probe calls the sorts' own entry functions, on a context of its own, whose scratch does not
+// count against the caller's budget.
+int probe_shipping_kernels(int device, int* ok) {
+  *ok = 0;
+  hpcs_config cfg;
+  hpcs_config_default(&cfg);
+  cfg.rank_mode = 1;  // (no probe for this one)
+  hpcs_ctx* ctx = nullptr;
+  int rc = hpcs_ctx_create(device, &cfg, &ctx);
+  if (rc != HPCS_OK) return rc;
+  ctx->rank_mode = RANK_ORDERED_ATOMIC;
+  const int64_t most = std::max(int64_t(2) << 20, int64_t(ctx->sms) * 512 * 32 + 12345);
   uint32_t *keys = nullptr, *items = nullptr, *bad = nullptr;
-  cudaError_t e = cudaMalloc(&keys, size_t(sizes[1]) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&items, size_t(sizes[1]) * 4);
+  cudaError_t e = cudaMalloc(&keys, size_t(most) * 4);
+  if (e == cudaSuccess) e = cudaMalloc(&items, size_t(most) * 4);
   if (e == cudaSuccess) e = cudaMalloc(&bad, 4);
   if (e == cudaSuccess) e = cudaMemset(bad, 0, 4);
-  int rc = e == cudaSuccess ? HPCS_OK : cuda_fail(e, "probe buffers");
-  const int saved_mode = ctx->rank_mode;
-  const int saved_scheme = ctx->cfg.pass_scheme;
-  ctx->rank_mode = RANK_ORDERED_ATOMIC;
+  if (e != cudaSuccess) rc = cuda_fail(e, "probe buffers");
   cudaStream_t s = ctx->stream;
-  struct Probe {
-    int scheme;
-    int64_t n;
+  auto fill = [&](int64_t n, uint32_t* it, uint32_t values) {
+    probe_fill_kernel<<<ctx->sms * 4, 256, 0, s>>>(keys, it, n, values);
+    if ((e = cudaGetLastError()) != cudaSuccess) rc = cuda_fail(e, "probe fill");
   };
-  for (const Probe& pr : {Probe{HPCS_PASSES_CHUNKED, sizes[0]}, Probe{HPCS_PASSES_LOOKBACK, sizes[0]},
-                          Probe{HPCS_PASSES_LOOKBACK, sizes[1]}, Probe{HPCS_PASSES_LOOKBACK, sizes[2]}}) {
-    ctx->cfg.pass_scheme = pr.scheme;
-    for (uint32_t values : {20u, 3u}) {
-      for (int with_items = 0; with_items < 2 && rc == HPCS_OK; with_items++) {
-        uint32_t* it = with_items ? items : nullptr;
-        probe_fill_kernel<<<ctx->sms * 4, 256, 0, s>>>(keys, it, pr.n, values);
-        if ((e = cudaGetLastError()) != cudaSuccess) rc = cuda_fail(e, "probe fill");
+  auto check = [&](int64_t n, uint32_t* it) {
+    if (rc != HPCS_OK) return;
+    probe_check_kernel<<<ctx->sms * 4, 256, 0, s>>>(keys, it, n, bad);
+    if ((e = cudaGetLastError()) != cudaSuccess) rc = cuda_fail(e, "probe check");
+  };
+  for (uint32_t values : {20u, 4u, 3u}) {
+    for (int with_items = 0; with_items < 2; with_items++) {
+      uint32_t* it = with_items ? items : nullptr;
+      for (const ProbeSort& pr : probe_sorts(ctx->sms, with_items != 0)) {
+        if (rc != HPCS_OK) break;
+        ctx->cfg.pass_scheme = pr.scheme;
+        fill(pr.n, it, values);
         if (rc == HPCS_OK)
           rc = with_items ? enqueue_sort<uint32_t, KIND_UNSIGNED, uint32_t>(ctx, keys, items, pr.n, s)
                           : enqueue_sort<uint32_t, KIND_UNSIGNED, NoValue>(ctx, keys, nullptr, pr.n, s);
-        if (rc == HPCS_OK) {
-          probe_check_kernel<<<ctx->sms * 4, 256, 0, s>>>(keys, it, pr.n, bad);
-          if ((e = cudaGetLastError()) != cudaSuccess) rc = cuda_fail(e, "probe check");
-        }
+        check(pr.n, it);
       }
     }
-  }
-  // the one-launch sort of small arrays (cluster_sort.cuh), taken by the default scheme
-  ctx->cfg.pass_scheme = HPCS_PASSES_AUTO;
-  constexpr int64_t n_small = 100003;
-  for (uint32_t values : {20u, 3u}) {
-    for (int with_items = 0; with_items < 2 && rc == HPCS_OK; with_items++) {
-      uint32_t* it = with_items ? items : nullptr;
-      probe_fill_kernel<<<ctx->sms * 4, 256, 0, s>>>(keys, it, n_small, values);
-      if ((e = cudaGetLastError()) != cudaSuccess) rc = cuda_fail(e, "probe fill");
-      if (rc == HPCS_OK)
-        rc = with_items ? enqueue_sort<uint32_t, KIND_UNSIGNED, uint32_t>(ctx, keys, items, n_small, s)
-                        : enqueue_sort<uint32_t, KIND_UNSIGNED, NoValue>(ctx, keys, nullptr, n_small, s);
-      if (rc == HPCS_OK) {
-        probe_check_kernel<<<ctx->sms * 4, 256, 0, s>>>(keys, it, n_small, bad);
-        if ((e = cudaGetLastError()) != cudaSuccess) rc = cuda_fail(e, "probe check");
-      }
+    for (const ProbeSegment& pr : PROBE_SEGMENTS) {
+      if (rc != HPCS_OK) break;
+      ctx->seg_tuning_set = pr.narrow;  // (a table that is the caller's keeps the narrow shape)
+      const hpcs_segment seg{keys, pr.n, HPCS_U32, 0};
+      fill(pr.n, nullptr, values);
+      if (rc == HPCS_OK) rc = hpcs_sort_segmented_dev(ctx, &seg, 1, s);
+      check(pr.n, nullptr);
     }
   }
-  ctx->rank_mode = saved_mode;
-  ctx->cfg.pass_scheme = saved_scheme;
   uint32_t h = 1;
   if (rc == HPCS_OK && (e = cudaStreamSynchronize(s)) != cudaSuccess) rc = cuda_fail(e, "probe");
   if (rc == HPCS_OK && (e = cudaMemcpy(&h, bad, 4, cudaMemcpyDeviceToHost)) != cudaSuccess) rc = cuda_fail(e, "probe");
@@ -238,6 +265,7 @@ int probe_shipping_kernels(hpcs_ctx* ctx, int* ok) {
   cudaFree(keys);
   cudaFree(items);
   cudaFree(bad);
+  hpcs_ctx_destroy(ctx);
   *ok = rc == HPCS_OK && h == 0;
   return rc;
 }
@@ -709,6 +737,24 @@ const char* hpcs_status_string(int status) {
   }
 }
 
+int hpcs_sort_shape(int key_bytes, int has_items, int pass_scheme, int64_t n, int sms) {
+  constexpr int ORDERED = RANK_ORDERED_ATOMIC;
+  if (pass_scheme == HPCS_PASSES_CHUNKED) return 0;
+  const int small = key_bytes == 8 ? (has_items ? cluster_kpt<uint64_t, uint32_t, ORDERED>(n) : cluster_kpt<uint64_t, NoValue, ORDERED>(n))
+                                   : (has_items ? cluster_kpt<uint32_t, uint32_t, ORDERED>(n) : cluster_kpt<uint32_t, NoValue, ORDERED>(n));
+  if (pass_scheme == HPCS_PASSES_AUTO && small) return (n <= int64_t(CS_NT) * small ? 200 : 300) + small;
+  return 100 + (key_bytes == 8 ? (has_items ? lookback_kpt<uint64_t, uint32_t, ORDERED>(n, sms) : lookback_kpt<uint64_t, NoValue, ORDERED>(n, sms))
+                               : (has_items ? lookback_kpt<uint32_t, uint32_t, ORDERED>(n, sms) : lookback_kpt<uint32_t, NoValue, ORDERED>(n, sms)));
+}
+
+int hpcs_probe_sort(int i, int has_items, int sms, int32_t* pass_scheme, int64_t* n) {
+  const std::vector<ProbeSort> v = probe_sorts(sms, has_items != 0);
+  if (i < 0 || i >= int(v.size()) || !pass_scheme || !n) return 0;
+  *pass_scheme = v[size_t(i)].scheme;
+  *n = v[size_t(i)].n;
+  return 1;
+}
+
 int hpcs_ctx_create(int device, const hpcs_config* cfg, hpcs_ctx** out) {
   if (!out) return fail(HPCS_ERR_NULL, "out is NULL");
   *out = nullptr;
@@ -761,7 +807,7 @@ int hpcs_ctx_create(int device, const hpcs_config* cfg, hpcs_ctx** out) {
       int& sp = shipping[device & 63];
       if (sp == 0) {
         int ok = 0;
-        if ((rc = probe_shipping_kernels(ctx, &ok)) != HPCS_OK) {
+        if ((rc = probe_shipping_kernels(device, &ok)) != HPCS_OK) {
           hpcs_ctx_destroy(ctx);
           return rc;
         }

@@ -384,17 +384,30 @@ int launch_cluster_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaS
   return HPCS_OK;
 }
 
+// Keys per thread of the one-launch small sort of n keys, 0 where n takes the large-array kernels.
+template <class U, class V, int MODE>
+inline int cluster_kpt(int64_t n) {
+  constexpr bool ONE = MODE == RANK_PEER_MASK;
+  constexpr int LARGEST = !ONE && sizeof(U) == 4 && std::is_same<V, NoValue>::value ? 32 : 16;
+  const int64_t per = n <= CS_SOLO_KEYS ? n : (n + CS_MAX_CTAS - 1) / CS_MAX_CTAS;  // keys a slice must hold
+  if (per > CS_NT * LARGEST) return 0;
+  if (ONE) return 16;
+  if (per <= CS_NT * 4 && n <= CS_SOLO_KEYS) return 4;
+  return per <= CS_NT * 8 ? 8 : per <= CS_NT * 16 ? 16 : LARGEST;
+}
+
 // A small sort in one cluster launch if n fits (else *done stays false).
 template <class U, int KIND, class V, int MODE>
 int enqueue_cluster_sort(hpcs_ctx* ctx, U* keys, uint32_t* vals, int64_t n, cudaStream_t s, bool* done) {
   constexpr bool ONE = MODE == RANK_PEER_MASK;
   constexpr int LARGEST = !ONE && sizeof(U) == 4 && std::is_same<V, NoValue>::value ? 32 : 16;
-  const int64_t per = n <= CS_SOLO_KEYS ? n : (n + CS_MAX_CTAS - 1) / CS_MAX_CTAS;  // keys a slice must hold
-  if (per <= CS_NT * 4 && n <= CS_SOLO_KEYS) return launch_cluster_sort<U, KIND, V, MODE, ONE ? 16 : 4>(ctx, keys, vals, n, s, done);
-  if (per <= CS_NT * 8) return launch_cluster_sort<U, KIND, V, MODE, ONE ? 16 : 8>(ctx, keys, vals, n, s, done);
-  if (per <= CS_NT * 16) return launch_cluster_sort<U, KIND, V, MODE, 16>(ctx, keys, vals, n, s, done);
-  if (per <= CS_NT * LARGEST) return launch_cluster_sort<U, KIND, V, MODE, LARGEST>(ctx, keys, vals, n, s, done);
-  return HPCS_OK;
+  switch (cluster_kpt<U, V, MODE>(n)) {
+    case 0: return HPCS_OK;
+    case 4: return launch_cluster_sort<U, KIND, V, MODE, ONE ? 16 : 4>(ctx, keys, vals, n, s, done);
+    case 8: return launch_cluster_sort<U, KIND, V, MODE, ONE ? 16 : 8>(ctx, keys, vals, n, s, done);
+    case 16: return launch_cluster_sort<U, KIND, V, MODE, 16>(ctx, keys, vals, n, s, done);
+    default: return launch_cluster_sort<U, KIND, V, MODE, LARGEST>(ctx, keys, vals, n, s, done);
+  }
 }
 
 // Whether the sort's rows (and its plan) fit the context's budget, or the slices it was lent.

@@ -268,6 +268,14 @@ typedef struct hpcs_seg_variant_info {
 int hpcs_seg_variants(hpcs_seg_variant_info* out, int capacity);
 /* Upper length limit of class c (-1 for the last, unbounded class; -2 if c is out of range). */
 int64_t hpcs_seg_class_limit(int c);
+
+/* The kernel shape that a plain sort takes with the ordered-atomic ranking on a device of `sms` SMs, as
+ * 100 x kind + keys per thread; kind 1: look-back passes, 2: one launch of one CTA, 3: one launch of one
+ * cluster (0, with no keys per thread: chunked passes, only where that scheme is given).  The probe that a
+ * process's first context runs covers every shape of 4-byte keys: hpcs_probe_sort gives its sort `i` (0 past
+ * the last one, else 1). */
+int hpcs_sort_shape(int key_bytes, int has_items, int pass_scheme, int64_t n, int sms);
+int hpcs_probe_sort(int i, int has_items, int sms, int32_t* pass_scheme, int64_t* n);
 int hpcs_ctx_get_seg_tuning(hpcs_ctx* ctx, hpcs_seg_tuning* out);
 /* HPCS_ERR_RANGE if a variant index is unknown or cannot hold the longest array of its class. */
 int hpcs_ctx_set_seg_tuning(hpcs_ctx* ctx, const hpcs_seg_tuning* tuning);

@@ -84,3 +84,18 @@ def test_still_refused(ctx):
             assert e.value.status == native.HPCS_ERR_OOM
         finally:
             c.close()
+
+
+def test_first_context_of_a_process_with_a_budget():
+    """The ranking probe of a process's first context has scratch of its own: a 12 MiB budget is enough for a
+    context and a million keys, whichever context comes first."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    code = ("import numpy as np\nfrom hpcsharp_b200 import native\nc = native.Context(0, pool_bytes=12 << 20)\n"
+            "a = np.random.default_rng(1).integers(0, 1 << 32, 1_000_000, dtype=np.uint32)\nw = np.sort(a)\nc.sort(a)\n"
+            "assert np.array_equal(a, w)\nassert c.rank_mode in (0, 1)\nc.close()\nprint('sorted')\n")
+    res = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert "sorted" in res.stdout, res.stderr[-2000:]
