@@ -16,8 +16,10 @@
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <fstream>
 #include <functional>
 #include <mutex>
+#include <string>
 #include <system_error>
 #include <thread>
 #include <vector>
@@ -116,6 +118,7 @@ class CopyPool {
         _mm_pause();
 #endif
       }
+      std::this_thread::yield();  // where threads outnumber CPUs the one looked for may need this one
     } while (std::chrono::steady_clock::now() < until);
     return false;
   }
@@ -153,13 +156,48 @@ class CopyPool {
   size_t bytes_ = 0;
 };
 
-// Copy threads: the host's hardware threads, at most 8.  Measured on a 16-core host of a B200
+// CPUs that the process may use at a time by its control group's quota (cgroup v2, its group and every group
+// above; else v1), at least 1; no quota: 0.  `root` and `self` stand for /sys/fs/cgroup and /proc/self/cgroup.
+inline int quota_cpus(const std::string& root, const std::string& self) {
+  int least = 0;
+  auto note = [&](double quota, double period) {
+    if (quota <= 0 || period <= 0) return;
+    const int cpus = std::max(1, int(quota / period + 0.5));
+    least = least ? std::min(least, cpus) : cpus;
+  };
+  auto number = [](const std::string& path) {
+    double v = 0;
+    std::ifstream(path) >> v;
+    return v;
+  };
+  std::string line, group;
+  for (std::ifstream f(self); std::getline(f, line);)
+    if (line.compare(0, 3, "0::") == 0) group = line.substr(3);
+  for (;;) {
+    while (!group.empty() && group.back() == '/') group.pop_back();
+    std::ifstream f(root + group + "/cpu.max");  // "quota period", or "max period"
+    double quota = 0, period = 0;
+    if (f >> quota >> period) note(quota, period);
+    if (group.empty()) break;
+    group.erase(group.rfind('/') == std::string::npos ? 0 : group.rfind('/'));
+  }
+  note(number(root + "/cpu/cpu.cfs_quota_us"), number(root + "/cpu/cpu.cfs_period_us"));
+  return least;
+}
+
+// Copy threads: the host's hardware threads, at most 8, and no more than a CPU quota allows (the threads look
+// for work between chunks: more of them than CPUs wait for one another, and spend the quota).  Measured on a 16-core host of a B200
 // node (1 GiB through 16 MiB chunks): pageable -> pinned 10 GB/s on one thread, 46-48 GB/s on
 // 8, 44-45 GB/s on 16; pinned -> pageable with streaming stores 61 GB/s on 8 and 51 GB/s on
 // 16.  The DMA engine moves about 56 GB/s each way over the host link.
 inline int stager_threads() {
-  const unsigned hw = std::thread::hardware_concurrency();
-  return int(std::max(1u, std::min(8u, hw ? hw : 1u)));
+  static const int threads = [] {
+    const unsigned hw = std::thread::hardware_concurrency();
+    const int quota = quota_cpus("/sys/fs/cgroup", "/proc/self/cgroup");
+    const int cpus = std::min(8, int(hw ? hw : 1u));
+    return std::max(1, quota ? std::min(cpus, quota) : cpus);
+  }();
+  return threads;
 }
 
 // Two rings, each allocated when first needed.  Arrays of 32 MiB and more run in 16 MiB chunks, where
