@@ -7,7 +7,7 @@
 //                                   Histogram.cs:1210-1248 (f32), :1250-1288 (f64)
 //   The transform is applied to the digit only; keys are moved as raw bits.
 // * PTX wrappers for mbarriers and 1-D bulk async copies (cp.async.bulk, no multicast),
-//   relaxed GPU-scope loads/stores for the decoupled look-back, and the global timer
+//   relaxed GPU-scope loads/stores for the look-back passes, and the global timer
 //   used to bound every spin.
 #pragma once
 #include <cstdint>
@@ -121,9 +121,6 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;

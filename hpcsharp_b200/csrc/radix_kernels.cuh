@@ -10,8 +10,8 @@
 //                       (ComputeStartOfBins, RadixSortLsd.cs:112-125), marks digit passes
 //                       whose keys all share one digit value as skippable (the idea of
 //                       RadixSortLsd.cs:2093-2117), and assigns ping-pong buffers.
-//   K3 digit passes     One launch per 8-bit digit: a single sweep with a decoupled look-back
-//                       (lookback_pass.cuh) or per-range passes without inter-CTA waiting
+//   K3 digit passes     One launch per 8-bit digit: a single sweep whose tiles' offsets one CTA
+//                       scans (lookback_pass.cuh) or per-range passes without inter-CTA waiting
 //                       (chunk_pass.cuh).  Ranking is stable (input order within a digit), so a
 //                       pass equals the reference's stable scatter (RadixSortLsdParallel.cs:96-135
 //                       with the bin-major / quantum-minor offsets of :49-94).
@@ -28,8 +28,10 @@ namespace hpcs {
 constexpr int RADIX = 256;
 constexpr int MAX_PASSES = 8;
 
-constexpr int64_t MAX_KEYS_PER_SORT = (int64_t(1) << 31) - 1;     // chunked passes: 32-bit positions
-constexpr int64_t MAX_KEYS_LOOKBACK = (int64_t(1) << 30) - 1;     // the forced look-back scheme's limit
+constexpr int64_t MAX_KEYS_PER_SORT = (int64_t(1) << 31) - 1;     // positions below 2^31
+// A forced look-back scheme has always refused more (its former passes had 30-bit prefixes); the present
+// ones have no such limit, and the default scheme runs them for every size.
+constexpr int64_t MAX_KEYS_LOOKBACK = (int64_t(1) << 30) - 1;
 struct NoValue {};
 
 // Per-sort control block in device memory (zeroed before K1).

@@ -123,8 +123,7 @@ typedef enum hpcs_kernel_class {
   HPCS_K_TOPK = 3,      /* radix select kernels */
   HPCS_K_SEGMENTED = 4, /* batched segmented sort kernels */
   HPCS_K_SHARD = 5,     /* sharded sort: partition of a shard (count, scan, scatter) */
-  HPCS_K_LOOKBACK = 6,  /* one 8-bit digit pass, decoupled look-back scheme (a launch whose
-                           scheme the histogram kernel did not choose returns at once) */
+  HPCS_K_LOOKBACK = 6,  /* one 8-bit digit pass in a single sweep, or a one-launch small sort */
   HPCS_K_CLASSES = 8
 } hpcs_kernel_class;
 
